@@ -42,7 +42,7 @@ namespace bpq4k {
 
 namespace {
 
-constexpr uint32_t kTokTile = 256;   // activation rows per CTA tile (= mma N)
+constexpr uint32_t kTokTile = 256;   // most activation rows per CTA tile (= mma N)
 constexpr uint32_t kKStep = 64;      // k per pipeline stage
 constexpr uint32_t kWaitLimit = 1u << 24;
 
@@ -58,6 +58,7 @@ struct PrefillArgs {
     // splitk_reduce_kernel adds the slices in a fixed order.  ksplit == 1: the kernel writes Y.
     uint32_t ksplit, bps;
     float* Ypart;
+    uint32_t tok_tile;  // activation rows of a tile of prefill_tc_kernel: a multiple of 16, at most kTokTile
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -103,9 +104,9 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* tma
 __device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr) {
     return (uint64_t)((smem_addr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
 }
-// Instruction descriptor, kind::f16: D = f32, A/B = f16 (0) or bf16 (1), both K-major, M = 128, N = 256.
-__device__ __forceinline__ constexpr uint32_t umma_idesc(bool bf16) {
-    return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((kTokTile >> 3) << 17) | ((128u >> 4) << 24);
+// Instruction descriptor, kind::f16: D = f32, A/B = f16 (0) or bf16 (1), both K-major, M = 128, N = n.
+__device__ __forceinline__ constexpr uint32_t umma_idesc(bool bf16, uint32_t n) {
+    return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 __device__ __forceinline__ void umma_f16(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
@@ -237,7 +238,7 @@ __global__ void __launch_bounds__(Plan<ROWS, PASSES, QT>::THREADS, 1) prefill_tc
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + P::STAGES * P::STAGE_BYTES + 2u * P::STAGES * 8u + 32u);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t n0 = blockIdx.x * ROWS, tok0 = blockIdx.y * kTokTile;
+    const uint32_t n0 = blockIdx.x * ROWS, tok0 = blockIdx.y * a.tok_tile;
     const uint32_t blk0 = blockIdx.z * a.bps;                          // first super-block of this K slice
     const uint32_t blk1 = min(a.K / kQK, blk0 + a.bps);
     const uint32_t nkb = (blk1 - blk0) * 4u;                           // pipeline iterations (64 k each)
@@ -273,14 +274,14 @@ __global__ void __launch_bounds__(Plan<ROWS, PASSES, QT>::THREADS, 1) prefill_tc
             for (uint32_t kb = 0; kb < nkb; kb++) {
                 const uint32_t s = kb % P::STAGES, it = kb / P::STAGES;
                 if (it > 0 && !wait_bar(empty_bar(s), (it - 1) & 1u, abort_flag, a.status)) break;
-                mbar_expect_tx(full_bar(s), P::NV * P::B_BYTES);
+                mbar_expect_tx(full_bar(s), P::NV * a.tok_tile * 128u);
                 for (uint32_t v = 0; v < P::NV; v++) tma_load_2d(b_tile(s, v), &a.tmap_x[v], kbase + kb * kKStep, tok0, full_bar(s));
             }
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer ----------------
         if (lane == 0) {
-            constexpr uint32_t idesc = umma_idesc(BF16);
+            const uint32_t idesc = umma_idesc(BF16, a.tok_tile);
             bool ok = true;
             for (uint32_t kb = 0; kb < nkb && ok; kb++) {
                 const uint32_t s = kb % P::STAGES, it = kb / P::STAGES;
@@ -593,12 +594,12 @@ __global__ void __launch_bounds__(Plan<ROWS, PASSES, QT>::THREADS, 1) prefill_tc
             // the warps of one quadrant share the accumulators and, when there are more warps than accumulators, the columns
             constexpr uint32_t NACC = (uint32_t)ROWS / 128u, NCP = P::DEQ_WARPS / 4u / NACC;
             const uint32_t accum = (dw / 4u) % NACC;        // which 128-row accumulator
-            const uint32_t cpart = (dw / 4u) / NACC;        // which run of kTokTile / NCP columns
+            const uint32_t cpart = (dw / 4u) / NACC;        // which of every NCP runs of 32 columns
             const uint32_t row = n0 + accum * 128u + quad * 32u + lane;
             const float bias = (a.ksplit == 1 && a.bias && row < a.N) ? a.bias[row] : 0.f;
             float* Yout = a.ksplit == 1 ? a.Y : a.Ypart + (uint64_t)blockIdx.z * a.M * a.N;
-            for (uint32_t c0 = cpart * (kTokTile / NCP); c0 < (cpart + 1u) * (kTokTile / NCP); c0 += 32) {
-                if (tok0 + c0 >= a.M) break;
+            const uint32_t tok_end = min(a.M, tok0 + a.tok_tile);
+            for (uint32_t c0 = cpart * 32u; tok0 + c0 < tok_end; c0 += NCP * 32u) {
                 uint32_t v[32];
                 tmem_ld32(tmem_base + ((quad * 32u) << 16) + accum * kTokTile + c0, v);
                 if constexpr (PASSES == 3) {  // add the cross-term accumulator
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(Plan<ROWS, PASSES, QT>::THREADS, 1) prefill_tc
 #pragma unroll
                     for (uint32_t t = 0; t < 32; t++) {
                         const uint32_t tok = tok0 + c0 + t;
-                        if (tok < a.M) Yout[(uint64_t)tok * a.N + row] = __uint_as_float(v[t]) + bias;
+                        if (tok < tok_end) Yout[(uint64_t)tok * a.N + row] = __uint_as_float(v[t]) + bias;
                     }
                 }
             }
@@ -1155,7 +1156,7 @@ cudaError_t launch_tc(const PrefillArgs& pa, cudaStream_t stream) {
     if (cudaError_t e = kcfg.prepare(reinterpret_cast<const void*>(prefill_tc_kernel<ROWS, PASSES, BF16, QT>), P::THREADS,
                                      P::SMEM_BYTES, nullptr))
         return e;
-    const dim3 grid((pa.N + ROWS - 1) / ROWS, (pa.M + kTokTile - 1) / kTokTile, pa.ksplit);
+    const dim3 grid((pa.N + ROWS - 1) / ROWS, (pa.M + pa.tok_tile - 1) / pa.tok_tile, pa.ksplit);
     prefill_tc_kernel<ROWS, PASSES, BF16, QT><<<grid, P::THREADS, P::SMEM_BYTES, stream>>>(pa);
     return cudaGetLastError();
 }
@@ -1201,6 +1202,12 @@ cudaError_t launch_tc_pair(const PrefillArgs& pa, cudaStream_t stream) {
 static int variant_of(int mode, uint32_t M) {
     const int v = (mode & 15) == 0 ? 0 : mode >> 4;
     return (v == 1 && M <= kTokTile) ? 0 : v;  // a pair's tile is 512 activation rows: nothing to share below 257
+}
+// Activation rows per tile: the rows are shared out evenly over as few tiles as possible, in steps of 16 (the mma's
+// granularity), so that no tile multiplies padding: 200 rows are one tile of 208, 300 rows two of 160.
+static uint32_t choose_tok_tile(uint32_t M) {
+    const uint32_t tiles = (M + kTokTile - 1u) / kTokTile;
+    return ((M + tiles - 1u) / tiles + 15u) & ~15u;
 }
 static uint32_t choose_ksplit(uint32_t M, uint32_t N, uint32_t K, int mode_v, int sm_count) {
     const int mode = mode_v & 15, variant = variant_of(mode_v, M);
@@ -1261,13 +1268,14 @@ cudaError_t launch_prefill_tc(const MatmulArgs& m, int mode_v, void* scratch, si
     pa.K = m.K;
     pa.w_row_bytes = m.w_row_bytes;
     pa.status = status_dev;
+    pa.tok_tile = choose_tok_tile(m.M);
     pa.ksplit = choose_ksplit(m.M, m.N, m.K, mode_v, sm_count);
     pa.bps = (m.K / kQK + pa.ksplit - 1) / pa.ksplit;
     pa.Ypart = reinterpret_cast<float*>(lo + (mode == 0 ? (((size_t)m.M * m.K * 2u + 255u) & ~(size_t)255u) : 0));
     for (int v = 0; v < (mode == 0 ? 2 : 1); v++) {
         const cuuint64_t gdim[2] = {(cuuint64_t)m.K, (cuuint64_t)m.M};
         const cuuint64_t gstride[1] = {(cuuint64_t)m.K * 2u};
-        const cuuint32_t box[2] = {kKStep, variant ? 128u : kTokTile};  // pairs and the tensor-memory form load 128 activation rows per copy
+        const cuuint32_t box[2] = {kKStep, variant ? 128u : pa.tok_tile};  // pairs and the tensor-memory form load 128 activation rows per copy
         const cuuint32_t estr[2] = {1u, 1u};
         const CUresult r = enc(&pa.tmap_x[v], CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, v == 0 ? hi : lo, gdim, gstride, box, estr,
                                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
