@@ -22,6 +22,19 @@ struct bpq4k_context {
     int prefill_variant = 0;  // BPQ4K_OPT_PREFILL_VARIANT
     int prefill_arg() const { return prefill_mode | (prefill_variant << 4); }  // what the launcher takes
     int prefill_min_m = 25;  // four 8-row slabs of the streaming kernel cost as much as one tensor-core pass
+    int rows_min_m = 9;  // smallest M of the several-rows kernel (takes_rows_kernel)
+    // its workspaces, one per stream that uses it (overlapping calls on two streams must not share one): counters and
+    // the buffer of calls of up to kRowsFixedM rows; two are allocated with the handle (a program's stream and the one it
+    // captures graphs on), two more when needed
+    static constexpr uint32_t kRowsFixedM = 64;
+    static constexpr size_t kRowsCounterBytes = 1024;
+    struct RowsWorkspace {
+        uint8_t* mem = nullptr;
+        cudaStream_t stream = nullptr;
+        bool assigned = false;
+    };
+    static constexpr uint32_t kRowsWorkspaces = 4;
+    RowsWorkspace rows_ws[kRowsWorkspaces];
     uint64_t launches = 0;
     // staging for the *_host entry point
     float* stage_x = nullptr;
@@ -148,12 +161,90 @@ constexpr uint32_t kStreamMaxM = 16;  // rows of X one streaming launch can cove
 // two slabs of 8 read from shared memory: 304 against 199 us on 128256 x 4096).
 inline uint32_t stream_slab_rows(uint32_t K) { return (uint64_t)K * 16u * 4u <= 132u * 1024u ? 16u : 8u; }
 
+int alloc_rows_workspace(bpq4k_context::RowsWorkspace& w) {
+    const size_t bytes = bpq4k_context::kRowsCounterBytes + rows_buffer_bytes(bpq4k_context::kRowsFixedM, kRowsMaxK);
+    if (cudaMalloc(reinterpret_cast<void**>(&w.mem), bytes) == cudaSuccess && cudaMemset(w.mem, 0, bpq4k_context::kRowsCounterBytes) == cudaSuccess)
+        return BPQ4K_OK;
+    cudaGetLastError();
+    if (w.mem) cudaFree(w.mem);
+    w.mem = nullptr;
+    return BPQ4K_ERR_ALLOC;
+}
+
+// The several-rows kernel's workspace for calls on `st`; null: none left (or none can be allocated while `st` is being
+// captured), and the caller takes the other kernels.
+uint8_t* rows_workspace(bpq4k_context* h, cudaStream_t st) {
+    for (auto& w : h->rows_ws)
+        if (w.assigned && w.stream == st) return w.mem;
+    for (auto& w : h->rows_ws) {
+        if (w.assigned) continue;
+        if (!w.mem) {
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+                cudaGetLastError();
+                return nullptr;
+            }
+            if (alloc_rows_workspace(w) != BPQ4K_OK) return nullptr;
+        }
+        w.assigned = true;
+        w.stream = st;
+        return w.mem;
+    }
+    return nullptr;
+}
+
+// Which Q4_K / Q5_K calls take the several-rows kernel.  Below rows_min_m (9) the streaming kernel is as fast: it reads
+// the weights once for 8 rows (128256 x 4096: 8 rows 101 us against 105 here, 9 rows 150 against 105); below prefill_min_m it stops at 24 rows (a caller who moves the tensor-core threshold up asks for the streaming
+// kernel); at and above the threshold it keeps the float accuracy of the F16X3 mode, so the 16-bit modes, which ask for
+// less, stay with their own kernel.  More than 32 rows of a short K stay with the prefill kernel: from 33 rows on high and
+// low halves share an accumulator, 5.7e-7 of error at any K; the prefill kernel has 3.5e-7 at K = 256, 1.2e-6 at K = 1024.
+bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a) {
+    if (h->gemv_variant != BPQ4K_GEMV_AUTO || a.n_slots || a.n_peers || !aligned16(a.X)) return false;
+    if (a.M < (uint32_t)h->rows_min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u)) return false;
+    return a.M >= (uint32_t)h->prefill_min_m ? h->prefill_mode == BPQ4K_PREFILL_F16X3 : a.M <= 24u;
+}
+
+// One call of the several-rows kernel.  cudaErrorInvalidValue: it cannot serve the call (form, shape or memory), and the
+// caller takes the other kernels.  More than kRowsFixedM rows use the handle's scratch as the prefill kernel does.
+// `owner`: the stream in whose order the call runs, where that is not `st` itself.
+cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, cudaStream_t owner, int qtype, int* launches) {
+    if (!takes_rows_kernel(h, a)) return cudaErrorInvalidValue;
+    uint8_t* ws = rows_workspace(h, owner);
+    if (!ws) return cudaErrorInvalidValue;
+    void* buffer = ws + bpq4k_context::kRowsCounterBytes;
+    const size_t need = rows_buffer_bytes(a.M, a.K);
+    size_t have = rows_buffer_bytes(bpq4k_context::kRowsFixedM, kRowsMaxK);
+    if (a.M > bpq4k_context::kRowsFixedM) {
+        if (need > h->scratch_bytes) {
+            // nothing may be allocated while the stream is being captured; the prefill kernel may need less
+            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+            if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+                ensure_bytes(h, &h->scratch, &h->scratch_bytes, need) != BPQ4K_OK) {
+                cudaGetLastError();
+                return cudaErrorInvalidValue;
+            }
+        }
+        buffer = h->scratch;
+        have = h->scratch_bytes;
+    }
+    return launch_rows_tc(a, reinterpret_cast<uint32_t*>(ws), buffer, have, h->dev_status, h->sm_count, &h->tmaps, !h->tune.no_pdl,
+                          st, launches, qtype);
+}
+
 // Kernel selection.  FP32: always the float kernel.  STREAM / AUTO: the streaming
 // kernel, X walked in slabs of 8 rows (each slab re-reads the weights, as the
 // reference's batched8 shader does per 8 rows).
-int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
+// `owner`: the stream in whose order the call runs, where that is not `st` itself.
+int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, cudaStream_t owner) {
     int launches = 0;
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = run_rows(h, a, st, owner, BPQ4K_TYPE_Q4_K, &launches);
+    if (e != cudaErrorInvalidValue) {
+        h->launches += (uint64_t)launches;
+        if (e == cudaSuccess) return BPQ4K_OK;
+        cudaGetLastError();
+        return cuda_fail(h, e, "matmul launch");
+    }
+    e = cudaSuccess;
     if (h->gemv_variant == BPQ4K_GEMV_FP32) {
         e = launch_gemv_fp32(a, st, &launches);
     } else if (!a.n_slots && a.M >= (uint32_t)h->prefill_min_m && h->gemv_variant == BPQ4K_GEMV_AUTO) {
@@ -241,9 +332,14 @@ int bpq4k_create(int device, bpq4k_handle_t* out) {
             e2 = cudaMalloc(&h->scratch, 4u << 20);
             if (e2 == cudaSuccess) h->scratch_bytes = 4u << 20;
         }
+        for (int i = 0; i < 2 && e2 == cudaSuccess; i++)
+            if (alloc_rows_workspace(h->rows_ws[i]) != BPQ4K_OK) e2 = cudaErrorMemoryAllocation;
         if (e2 != cudaSuccess) {
             cudaGetLastError();
             if (h->dev_status) cudaFree(h->dev_status);
+            if (h->scratch) cudaFree(h->scratch);
+            for (auto& w : h->rows_ws)
+                if (w.mem) cudaFree(w.mem);
             delete h;
             return BPQ4K_ERR_ALLOC;
         }
@@ -261,6 +357,8 @@ int bpq4k_destroy(bpq4k_handle_t h) {
         if (h->scratch) cudaFree(h->scratch);
         if (h->dev_status) cudaFree(h->dev_status);
         if (h->tune.stamps) cudaFree(h->tune.stamps);
+        for (auto& w : h->rows_ws)
+            if (w.mem) cudaFree(w.mem);
         for (uint32_t i = 0; i < h->n_retired; i++) cudaFree(h->retired[i]);
         if (h->batch_exec) cudaGraphExecDestroy(h->batch_exec);
         if (h->batch_stream) cudaStreamDestroy(h->batch_stream);
@@ -290,6 +388,10 @@ int bpq4k_set_option(bpq4k_handle_t h, int option, int value) {
         case BPQ4K_OPT_PREFILL_MIN_M:
             if (value < 1) return fail(h, BPQ4K_ERR_INVALID_ARG, "prefill_min_m must be >= 1");
             h->prefill_min_m = value;
+            return BPQ4K_OK;
+        case BPQ4K_OPT_ROWS_MIN_M:
+            if (value < 1) return fail(h, BPQ4K_ERR_INVALID_ARG, "rows_min_m must be >= 1");
+            h->rows_min_m = value;
             return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_WARPS:
             if (value < 0 || value > 16) return fail(h, BPQ4K_ERR_INVALID_ARG, "stream warps must be 0..16");
@@ -377,6 +479,7 @@ int bpq4k_get_option(bpq4k_handle_t h, int option, int* value) {
         case BPQ4K_OPT_PREFILL_VARIANT: *value = h->prefill_variant; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_STAMPS: *value = (int)h->tune.stamp_launches; return BPQ4K_OK;
         case BPQ4K_OPT_PREFILL_MIN_M: *value = h->prefill_min_m; return BPQ4K_OK;
+        case BPQ4K_OPT_ROWS_MIN_M: *value = h->rows_min_m; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_WARPS: *value = (int)h->tune.warps; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_KSPLIT: *value = (int)h->tune.wk; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_STAGE_BLOCKS: *value = (int)h->tune.cb; return BPQ4K_OK;
@@ -505,7 +608,7 @@ int bpq4k_matmul_f32(bpq4k_handle_t h, const float* X, const void* W, const floa
     a.N = N;
     a.K = K;
     a.w_row_bytes = (uint64_t)rowStrideWords * 4u;
-    return run_matmul(h, a, static_cast<cudaStream_t>(stream));
+    return run_matmul(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream));
 }
 
 // ---- Q5_K / Q6_K siblings ----------------------------------------------------
@@ -618,6 +721,15 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
     a.w_row_bytes = (uint64_t)rowStrideWords * 4u;
     int launches = 0;
     cudaError_t e = cudaErrorInvalidValue;
+    if (qtype == BPQ4K_TYPE_Q5_K) {
+        e = run_rows(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream), qtype, &launches);
+        if (e != cudaErrorInvalidValue) {
+            h->launches += (uint64_t)launches;
+            if (e == cudaSuccess) return BPQ4K_OK;
+            cudaGetLastError();
+            return cuda_fail(h, e, "matmul launch");
+        }
+    }
     // many rows of Q5_K or padded Q6_K: the tensor-core kernel, as for Q4_K
     const bool tensor_cores = (qtype == BPQ4K_TYPE_Q5_K || qtype == BPQ4K_TYPE_Q6_K_PADDED) && h->gemv_variant == BPQ4K_GEMV_AUTO &&
                               aligned16(X) && M >= (uint32_t)h->prefill_min_m;
@@ -759,7 +871,7 @@ int bpq4k_matmul_moe_f32(bpq4k_handle_t h, const float* X, const void* W, const 
     a.x_rows = x_rows;
     a.n_slots = nSlots;
     a.w_total_rows = wRows;
-    return run_matmul(h, a, static_cast<cudaStream_t>(stream));
+    return run_matmul(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream));
 }
 
 int bpq4k_kq_matmul_moe_f32(bpq4k_handle_t h, int qtype, const float* X, const void* W, const float* bias, float* Y,
@@ -914,7 +1026,7 @@ int bpq4k_matmul_host_f32(bpq4k_handle_t h, const float* X_host, const void* W_d
     a.N = N;
     a.K = K;
     a.w_row_bytes = (uint64_t)rowStrideWords * 4u;
-    if (int s = run_matmul(h, a, st)) return s;
+    if (int s = run_matmul(h, a, st, st)) return s;
     e = cudaMemcpyAsync(Y_host, h->stage_y, yb, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "result read-back");
     e = cudaStreamSynchronize(st);
@@ -1157,7 +1269,7 @@ int bpq4k_matmul_host_batch_f32(bpq4k_handle_t h, const bpq4k_host_matmul* items
             a.N = it.N;
             a.K = it.K;
             a.w_row_bytes = (uint64_t)it.rowStrideWords * 4u;
-            if (int s = run_matmul(h, a, s_)) return s;
+            if (int s = run_matmul(h, a, s_, st)) return s;  // (recorded on the handle's own stream, replayed in the order of st)
             xo += ((size_t)it.M * it.K * 4u + 255u) & ~(size_t)255u;
             yo += ((size_t)it.M * it.N * 4u + 255u) & ~(size_t)255u;
         }
@@ -1185,7 +1297,7 @@ int bpq4k_matmul_host_batch_f32(bpq4k_handle_t h, const bpq4k_host_matmul* items
     uint64_t key = 1469598103934665603ull;
     key = fnv1a(key, items, sizeof(bpq4k_host_matmul) * count);
     key = fnv1a(key, &h->tune, sizeof(h->tune));
-    const int opts[3] = {h->gemv_variant, h->prefill_arg(), h->prefill_min_m};
+    const int opts[4] = {h->gemv_variant, h->prefill_arg(), h->prefill_min_m, h->rows_min_m};
     key = fnv1a(key, opts, sizeof(opts));
     const void* bufs[3] = {h->stage_x, h->stage_y, h->scratch};  // the graph holds these addresses
     key = fnv1a(key, bufs, sizeof(bufs));

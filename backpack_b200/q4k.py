@@ -39,6 +39,7 @@ OPT_STREAM_PREWAIT_STAGES = 18
 OPT_STREAM_CLUSTER = 20
 OPT_STREAM_STAGING_WARPS = 21
 OPT_PREFILL_VARIANT = 23
+OPT_ROWS_MIN_M = 25
 OPT_STREAM_STAMPS = 24
 PREFILL_ONE_CTA, PREFILL_CTA_PAIR, PREFILL_TMEM_WEIGHTS = 0, 1, 2
 OPT_STREAM_UNIT_ROWS = 19

@@ -1,0 +1,159 @@
+"""Several activation rows in one pass over the weights (q4k_rows_tc.cu): Q4_K and Q5_K, against the float expectation in 64 bits."""
+import numpy as np
+import pytest
+
+from backpack_b200 import q4k, synth
+from oracle import q4k_oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    import backpack_b200 as bp
+
+    c = bp.Q4KContext(0)
+    c.set_option(q4k.OPT_ROWS_MIN_M, 2)   # (also the row counts that the streaming kernel serves by default)
+    yield c
+    c.close()
+
+
+def make(qtype, N, K, seed):
+    """(raw file bytes, dequantised weights in 64 bits)"""
+    if qtype == q4k.Q4_K:
+        raw = synth.make_q4k_weights(N, K, seed)
+        return raw, orc.dequant(raw, N, K).reshape(N, K).astype(np.float64)
+    raw = synth.make_kq_weights(q4k.Q5_K, N, K, seed)
+    return raw, orc.kq_dequant(orc.Q5_K, raw, N, K).reshape(N, K).astype(np.float64)
+
+
+def upload(ctx, qtype, raw, N, K):
+    return ctx.upload(q4k.pack_q4k(raw, N, K) if qtype == q4k.Q4_K else q4k.pack_kq(q4k.Q5_K, raw, N, K))
+
+
+def close(y, x, w64, bias=None):
+    """Bound: the activations carry 22 bits (2^-23 of the largest of a row), a super-block's products accumulate in
+    float with truncation (16 steps of 2^-23 at most), the super-blocks in float: 3e-6 of |x| |w| summed covers all."""
+    x64 = x.astype(np.float64)
+    want = x64 @ w64.T + (0.0 if bias is None else bias.astype(np.float64))
+    scale = np.sqrt((x64**2) @ (w64.T**2)) + np.abs(want) + 1e-30
+    assert np.isfinite(y).all()
+    rel = np.linalg.norm(y - want) / np.linalg.norm(want)
+    assert np.abs((y - want) / scale).max() <= 6e-6 * np.sqrt(np.log2(w64.shape[1])) and rel <= 4e-6, (np.abs((y - want) / scale).max(), rel)
+
+
+# every activation tile (8 .. 64), ragged rows of weights, one block to many, cut and whole tiles
+SHAPES = [(5, 1, 256), (8, 300, 1024), (9, 256, 512), (16, 4099, 1024), (17, 511, 768), (24, 1000, 2560), (25, 257, 4096),
+          (32, 640, 256), (33, 513, 1024), (48, 300, 1792), (49, 700, 1280), (64, 130, 4096), (64, 40000, 1024), (40, 300, 512)]
+
+
+@pytest.mark.parametrize("qtype", [q4k.Q4_K, q4k.Q5_K], ids=["q4_k", "q5_k"])
+@pytest.mark.parametrize("M,N,K", SHAPES)
+def test_rows_kernel_matches_64_bits(ctx, qtype, M, N, K):
+    import torch
+
+    raw, w64 = make(qtype, N, K, M + N)
+    x = synth.make_activations(M, K, M)
+    bias = np.linspace(-2, 2, N).astype(np.float32)
+    w = upload(ctx, qtype, raw, N, K)
+    xd, bd = torch.from_numpy(x).cuda(), torch.from_numpy(bias).cuda()
+    ctx.launch_count(reset=True)
+    y = ctx.matmul(xd, w, bias=bd)
+    assert ctx.launch_count() in (2, 3)       # the activations' layout, the matmul, the sum of tiles cut into many segments
+    y2 = ctx.matmul(xd, w, bias=bd)
+    assert ctx.device_status() == 0
+    close(y.cpu().numpy(), x, w64, bias)
+    assert torch.equal(y, y2)                 # cut tiles are summed in a fixed order
+
+
+@pytest.mark.parametrize("M", [7, 20, 40, 64])
+def test_rows_kernel_range_of_activations_and_scales(ctx, M):
+    """Rows from 1e-30 to 1e30 in magnitude, a zero row, one outlier beside small values; super-blocks whose d is zero, or
+    tiny beside dmin, and blocks without a minimum."""
+    import torch
+
+    N, K = 300, 1024
+    raw = synth.make_q4k_weights(N, K, 5).reshape(N * (K // 256), 144).copy()
+    halves = raw[:, :4].view(np.float16)
+    halves[0::7, 0] = 0.0                     # d = 0: constant blocks
+    halves[1::7, 0] = 6e-8                    # the smallest half beside an ordinary dmin
+    halves[2::7, 1] = 0.0                     # no minimum
+    halves[3::7, :] = 0.0
+    raw = raw.reshape(-1)
+    w64 = orc.dequant(raw, N, K).reshape(N, K).astype(np.float64)
+    x = synth.make_activations(M, K, 6)
+    x *= (10.0 ** np.linspace(-30, 30, M)).astype(np.float32)[:, None]
+    x[M // 2] = 0.0
+    x[M // 3, 17] *= 1e6
+    w = ctx.upload(q4k.pack_q4k(raw, N, K))
+    y = ctx.matmul(torch.from_numpy(x).cuda(), w).cpu().numpy().astype(np.float64)
+    assert ctx.device_status() == 0
+    # The kernel splits a weight into sc*(q - 8) and a constant of its sub-block, so a weight that is small beside its
+    # sub-block's largest keeps that one's absolute error: 2^-23 of the activation (2^-39 of the row's largest where that
+    # is more), 16 truncated steps of 2^-23 at most.
+    wmax = np.repeat(np.abs(w64).reshape(N, K // 32, 32).max(axis=2), 32, axis=1)
+    for t in range(M):  # each row by itself: they differ by 60 orders of magnitude
+        x64 = x[t].astype(np.float64)
+        want = w64 @ x64
+        bound = 4e-6 * (wmax @ np.abs(x64)) + 2.0**-39 * np.abs(x64).max() * wmax.sum(axis=1) + 1e-37
+        assert np.all(np.abs(y[t] - want) <= bound), (t, np.max(np.abs(y[t] - want) / bound))
+
+
+def test_rows_kernel_not_finite_stays_in_its_row(ctx):
+    import torch
+
+    M, N, K = 12, 300, 512
+    raw, w64 = make(q4k.Q4_K, N, K, 9)
+    x = synth.make_activations(M, K, 10)
+    x[3, 100] = np.inf
+    x[7, 5] = np.nan
+    y = ctx.matmul(torch.from_numpy(x).cuda(), upload(ctx, q4k.Q4_K, raw, N, K)).cpu().numpy()
+    bad = np.array([3, 7])
+    good = np.setdiff1d(np.arange(M), bad)
+    assert not np.isfinite(y[bad]).any()
+    close(y[good], x[good], w64)
+
+
+def test_rows_kernel_threshold_streams_and_capture(ctx):
+    """Below the option's row count the streaming kernel runs; calls on several streams at once keep their own workspace;
+    a captured call replays."""
+    import torch
+
+    M, N, K = 12, 1000, 2048
+    raw, w64 = make(q4k.Q4_K, N, K, 11)
+    w = upload(ctx, q4k.Q4_K, raw, N, K)
+    xs = [synth.make_activations(M, K, 20 + i) for i in range(6)]
+    default = ctx.get_option(q4k.OPT_ROWS_MIN_M)
+    try:
+        ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)
+        close(ctx.matmul(torch.from_numpy(xs[0]).cuda(), w).cpu().numpy(), xs[0], w64)
+    finally:
+        ctx.set_option(q4k.OPT_ROWS_MIN_M, default)
+    xd = [torch.from_numpy(x).cuda() for x in xs]
+    ys = [torch.empty(M, N, device="cuda") for _ in xs]
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for x, y, s in zip(xd, ys, streams):
+            with torch.cuda.stream(s):
+                ctx.matmul(x, w, out=y)
+    torch.cuda.synchronize()
+    for x, y in zip(xs, ys):
+        close(y.cpu().numpy(), x, w64)
+    import backpack_b200 as bp
+
+    c = bp.Q4KContext(0)
+    try:
+        y = torch.empty(M, N, device="cuda")
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):             # the handle's first call: everything it needs was allocated with it
+            c.matmul(xd[0], w, out=y)
+        for x in (1, 2):
+            xd[0].copy_(xd[x])
+            g.replay()
+            torch.cuda.synchronize()
+            close(y.cpu().numpy(), xs[x], w64)
+        assert c.device_status() == 0
+        del g
+    finally:
+        c.close()
