@@ -198,17 +198,30 @@ uint8_t* rows_workspace(bpq4k_context* h, cudaStream_t st) {
 // kernel); at and above the threshold it keeps the float accuracy of the F16X3 mode, so the 16-bit modes, which ask for
 // less, stay with their own kernel.  More than 32 rows of a short K stay with the prefill kernel: from 33 rows on high and
 // low halves share an accumulator, 5.7e-7 of error at any K; the prefill kernel has 3.5e-7 at K = 256, 1.2e-6 at K = 1024.
-bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a) {
+bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a, int qtype) {
     if (h->gemv_variant != BPQ4K_GEMV_AUTO || a.n_slots || a.n_peers || !aligned16(a.X)) return false;
     if (a.M < (uint32_t)h->rows_min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u)) return false;
-    return a.M >= (uint32_t)h->prefill_min_m ? h->prefill_mode == BPQ4K_PREFILL_F16X3 : a.M <= 24u;
+    if (a.M < (uint32_t)h->prefill_min_m) return a.M <= 24u;
+    if (h->prefill_mode != BPQ4K_PREFILL_F16X3) return false;
+    // Against the prefill kernel (us, prefill | here).  To 96 rows here: 80 rows, 6144 x 4096 33 | 26, 128256 x 4096 350 | 195.
+    // To 128 rows where a CTA has enough units to pay for the cut tiles: 128 rows, 6144 x 4096 35 | 40, 4096 x 14336 58 | 54,
+    // 28672 x 4096 115 | 81.  To 256 rows the prefill kernel takes one tile and this one two, so only where its limit of
+    // 4096 k per slice makes it cut K: 200 rows, 4096 x 14336 74 | 81, 128256 x 4096 466 | 491, 57344 x 8192 529 | 400.
+    // Above here: 300 rows, 6144 x 4096 69 | 57; 512 rows, 6144 x 4096 96 | 93, 57344 x 8192 1183 | 951.
+    const uint64_t units = (uint64_t)((a.N + 255u) / 256u) * (a.K / BPQ4K_QK_K);
+    // Q5_K, whose larger blocks leave the raw ring one stage per row tile, only to 320 rows: 300 rows, 128256 x 4096
+    // 921 | 866; 512 rows 1251 | 1349, but 57344 x 8192 1188 | 1140.
+    const bool cut_k = a.K > 4096u && a.N >= 16384u;
+    if (a.M <= 96u) return true;
+    if (a.M > 256u) return qtype == BPQ4K_TYPE_Q4_K || a.M <= 320u || cut_k;
+    return a.M <= 128u ? units >= 800u : cut_k;
 }
 
 // One call of the several-rows kernel.  cudaErrorInvalidValue: it cannot serve the call (form, shape or memory), and the
 // caller takes the other kernels.  More than kRowsFixedM rows use the handle's scratch as the prefill kernel does.
 // `owner`: the stream in whose order the call runs, where that is not `st` itself.
 cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, cudaStream_t owner, int qtype, int* launches) {
-    if (!takes_rows_kernel(h, a)) return cudaErrorInvalidValue;
+    if (!takes_rows_kernel(h, a, qtype)) return cudaErrorInvalidValue;
     uint8_t* ws = rows_workspace(h, owner);
     if (!ws) return cudaErrorInvalidValue;
     void* buffer = ws + bpq4k_context::kRowsCounterBytes;

@@ -152,7 +152,7 @@ cudaError_t launch_prefill_tc(const MatmulArgs& a, int mode, void* scratch, size
 // Matmul of several activation rows, K up to 32768 (q4k_rows_tc.cu), two or three launches.  `counters`: 160 words that are zero
 // before the first call; `buffer`: rows_buffer_bytes() bytes; both serve one stream at a time.
 // cudaErrorInvalidValue: not a shape or form of this kernel.
-constexpr uint32_t kRowsMaxM = 64, kRowsMaxK = 32768;
+constexpr uint32_t kRowsMaxM = 16384, kRowsMaxK = 32768;
 size_t rows_buffer_bytes(uint32_t M, uint32_t K);
 cudaError_t launch_rows_tc(const MatmulArgs& a, uint32_t* counters, void* buffer, size_t buffer_bytes, int* status_dev,
                            int sm_count, TmapCache* tmaps, bool pdl, cudaStream_t stream, int* launches, int qtype = 12);

@@ -1,32 +1,34 @@
-// Q4_K / Q5_K matmul for a few to 64 activation rows on the 5th-generation tensor cores, weights read once.
+// Q4_K / Q5_K matmul of several activation rows on the 5th-generation tensor cores, at float accuracy in two half passes.
 //
 // The reference re-reads the weights for every 8 activation rows (q4k_matmul_batched8,
-// runtime/kernels/quant_kq/q4k_matmul_batched8.wgsl:9-23).  Here one pass over the weights serves all rows, and the
+// runtime/kernels/quant_kq/q4k_matmul_batched8.wgsl:9-23).  Here one pass over the weights serves up to 128 rows, and the
 // contraction is exact in the weights:
 //
 //   w = d*sc*q - dmin*mn = d * [ sc*(q - z) + (z*sc - (dmin/d)*mn) ]        (z = 8 for 4-bit codes, 16 for 5-bit codes)
 //
 // sc*(q - z) is an integer below 1024, exact in half precision, so ONE 16-bit weight operand serves an activation that
 // is split into two halves (x*2^e = Xh + Xl, 22 bits; e per activation row).  The bracket's second term is constant
-// over a sub-block of 32 weights: it multiplies the sub-block's sum of activations, which is one more k-step of 16
-// beside the four that a 64-weight group needs (high and low half of the constant, high and low half of the sum).  The
-// accumulator of a super-block (256 weights) is drained to registers, where d is applied in float: the tensor core
-// never accumulates over more than a super-block, so its truncating additions cost less than the float rounding.
+// over a sub-block of 32 weights: it multiplies the sub-block's mean activation, one more k-step of 16 per super-block
+// (high and low half of the eight constants).  The accumulator of a super-block (256 weights) is drained to registers,
+// where d is applied in float: the tensor core, whose additions truncate, never accumulates over more than a super-block.
+// Error against 64 bits 2.9e-7..3.7e-7 to 32 rows (streaming kernel 3.3e-7..4.5e-7), 5.7e-7..6.3e-7 above (prefill kernel
+// 1.2e-6..2.2e-6 from K = 1024 on).
 //
-// What bounds it: the weight stream, and now the instructions of the dequantising warps (3,500 cycles a unit of 256 rows x
-// 256 weights; 1,470 at the DRAM rate).  Measured on B200, whole call (was: streaming kernel in slabs, prefill kernel),
-// 128256 x 4096: 9 rows 105 us (150), 16 rows 108 (201), 24 rows 115 (302), 37 rows 147 (348), 64 rows 183 (347);
-// 1024 x 4096: 16 rows 12 us (18), 32 rows 12 (24).  Everything else is arranged around the weight stream:
+// What bounds it.  To 48 rows the instructions of the dequantising warps (3,300 cycles a unit of 256 rows x 256 weights,
+// 1,470 at the DRAM rate; ncu: issue slots 54 % busy, ALU 40 %); above, the hand-overs between dequantising, mma and drain
+// (T = 128: 7,200 cycles a unit, 4,350 of them mmas).  Whole call on B200, us, before | now (before: streaming kernel in
+// slabs, prefill kernel with three passes), 128256 x 4096: 16 rows 201 | 105, 24 rows 302 | 115, 37 rows 348 | 147, 64 rows
+// 348 | 159, 80 rows 350 | 195, 128 rows 387 | 267, 512 rows 1252 | 1166; 57344 x 8192, 512 rows: 1183 | 951.
 //   * the dequantised operand lives in TENSOR MEMORY (tcgen05.st, A operand of tcgen05.mma); through shared memory its
 //     write and re-read alone would cost 1.7 times the shared-memory bandwidth that streaming at the DRAM rate leaves;
 //   * a CTA takes 256 weight rows at a time (two 128-lane row tiles share every activation tile);
-//   * the work is one list of (row tile, super-block) units over at most one CTA per SM, cut into equal contiguous
-//     shares: every SM streams whatever the shape.  A row tile that is cut leaves partial sums in a workspace; the CTA
-//     that finishes last adds them in ascending order of k (deterministic).
+//   * the work is one list of (row tile, activation tile, super-block) units over at most one CTA per SM, cut into equal
+//     contiguous shares: every SM is busy whatever the shape.  A tile that is cut leaves partial sums in a workspace, which
+//     are added in ascending order of k (deterministic): by the CTA that finishes last, or by rows_reduce_kernel.
 //
-// Roles (20 warps): warp 0 TMA loads of raw super-blocks (box 128 rows x 1 block), warp 1 tensor memory and mma issue,
-// warp 2 bulk copies of the activation tiles (laid out by rows_pack_kernel exactly as the mma reads them), warps 4-19
-// dequantise and drain: row tile = (warp-4)/8, its 64-weight groups alternate between two sets of four warps.
+// Roles (20 warps): warp 0 TMA loads of raw super-blocks (box 128 rows x 1 block), warp 1 (and 3) mma issue, warp 2 bulk
+// copies of the activation tiles (laid out by rows_pack_kernel exactly as the mma reads them), warps 4-19 dequantise and
+// drain (RowsPlan says which does what).
 //
 // Every wait is bounded: on a time-out the role raises the CTA's abort flag and the device status word, waits return
 // at once from then on, the loops run out (so that all barriers stay matched), copies and mmas in flight are waited
@@ -43,24 +45,25 @@ namespace bpq4k {
 
 namespace {
 
-constexpr uint32_t kWaitLimit = 1u << 22;
+constexpr uint32_t kWaitLimit = 1u << 21;
+constexpr uint32_t kSuspendNs = 1000;                 // a waiting warp sleeps this long at most: polls take issue slots from the dequantising warps
 constexpr uint32_t kWorkers = 16;                     // warps that dequantise and drain
 constexpr uint32_t kThreads = (4 + kWorkers) * 32;
 constexpr uint32_t kTileRows = 256;                   // weight rows of a unit: two row tiles of 128 lanes
 constexpr uint32_t kASlotCols = 40;                   // tensor-memory columns of one dequantised group: 32 codes + 8 (constant term)
 
 // T: activation rows of the tile.
-//   up to 32   the high and the low halves of the activations are stacked into one mma of 2T columns (each has its own
-//              accumulator); above that they accumulate into the same T columns
-//   up to 64   two accumulators per row tile: the next super-block accumulates while the last one is drained
-//   above      one accumulator per row tile (tensor memory holds two tiles' accumulators and the operand ring); the
-//              second row tile runs two groups behind the first, so that one accumulates while the other is drained.
-//              The workers' partial sums take more registers than a launch of 20 warps leaves each: setmaxnreg.
+//   up to 32   the high and the low halves of the activations are stacked into one mma of 2T columns, each half with its
+//              own accumulator; above that they accumulate into the same T columns
+//   up to 48   two accumulators per row tile: the next super-block accumulates while the last is drained
+//   above      (WIDE) one accumulator per row tile (tensor memory holds two tiles' accumulators and the operand ring) and an issuing warp for each, the second two groups behind the
+//              first, so that one accumulates while the other is drained.  The T partial sums of a weight row fill a
+//              thread's registers, so eight warps dequantise and eight others drain: setmaxnreg 64 and 160.
 template <int T, int QT>
 struct RowsPlan {
     static constexpr bool STACK = T <= 32;
-    static constexpr uint32_t NBUF = T <= 64 ? 2u : 1u;
-    static constexpr uint32_t LAG = NBUF == 1u ? 2u : 0u;         // groups that the second row tile's mmas run behind
+    static constexpr bool WIDE = T > 48;
+    static constexpr uint32_t NBUF = WIDE ? 1u : 2u;
     static constexpr uint32_t N = STACK ? 2u * T : (uint32_t)T;   // columns of one accumulator
     static constexpr uint32_t ACC_COLS = 2u * NBUF * N;
     static constexpr uint32_t NA = (512u - ACC_COLS) / (2u * kASlotCols) > 5u ? 5u : (512u - ACC_COLS) / (2u * kASlotCols);
@@ -72,17 +75,15 @@ struct RowsPlan {
     // activation ring: a slot holds a super-block's four groups, or (one accumulator) one group
     static constexpr uint32_t BG = NBUF == 2u ? 4u : 1u;
     static constexpr uint32_t B_SLOT = (BG * G_BYTES + S_BYTES + 1023u) & ~1023u;
-    static constexpr uint32_t NB = T <= 8 ? 4u : T <= 24 ? 3u : T <= 64 ? 2u : T <= 96 ? 5u : 4u;
-    // barriers of the operand ring and of the accumulators: one set for both row tiles, or one each where the second lags
+    static constexpr uint32_t NB = T <= 8 ? 4u : T <= 24 ? 3u : T <= 48 ? 2u : T <= 96 ? 5u : 4u;
+    // barriers of the operand ring and of the accumulators: one set for both row tiles, or one each
     static constexpr uint32_t RB = NBUF == 2u ? 1u : 2u;
     static constexpr uint32_t BAR_BYTES = 1024u;
-    static constexpr uint32_t NR = (226u * 1024u - 1024u - BAR_BYTES - NB * B_SLOT) / RAW_BYTES > 10u
-                                       ? 10u : (226u * 1024u - 1024u - BAR_BYTES - NB * B_SLOT) / RAW_BYTES;
-    static constexpr uint32_t SMEM_BYTES = 1024u + NB * B_SLOT + NR * RAW_BYTES + BAR_BYTES;
-    // One accumulator: the worker drains between its two groups of a super-block, the first of which must find a free
-    // operand slot without the drained accumulator (groups 4k and 4k+1 after 4k-1 at the latest): NA >= 2, and the B ring
-    // holds the groups between the two row tiles beside one being loaded.
-    static_assert(NA >= 2 && NR >= 2 && NB >= (NBUF == 2u ? 2u : 2u + LAG), "rings too short");
+    static constexpr uint32_t S_RING = WIDE ? 4u * 256u * 4u : 0u;   // WIDE: the drain's scale of every weight row, four super-blocks deep
+    static constexpr uint32_t NR = (226u * 1024u - 1024u - BAR_BYTES - S_RING - NB * B_SLOT) / RAW_BYTES > 10u
+                                       ? 10u : (226u * 1024u - 1024u - BAR_BYTES - S_RING - NB * B_SLOT) / RAW_BYTES;
+    static constexpr uint32_t SMEM_BYTES = 1024u + NB * B_SLOT + NR * RAW_BYTES + BAR_BYTES + S_RING;
+    static_assert(NA >= 2 && NR >= 2 && NB >= 2, "rings too short");
 };
 
 struct RowsArgs {
@@ -113,10 +114,10 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity)
+        : "r"(bar), "r"(parity), "r"(kSuspendNs)
         : "memory");
     return ok;
 }
@@ -217,11 +218,99 @@ __device__ __forceinline__ uint32_t half2_bits(float a, float b) {
     const __half2 v = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&v);
 }
-// (1024 + 16 q) * (sc/16) - (64 + z) * sc = sc * (q - z), exact: `codes` holds 16 q in bits 4.. of both halves
-__device__ __forceinline__ uint32_t scale_codes(uint32_t codes, __half2 m, __half2 a) {
-    const uint32_t biased = codes | 0x64006400u;
+// (w & 0x00F000F0) | base in one instruction (the compiler makes two of the expression: 64 of 600 a warp and unit)
+__device__ __forceinline__ uint32_t codes_of(uint32_t w, uint32_t base) {
+    uint32_t r;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(w), "r"(0x00F000F0u), "r"(base));
+    return r;
+}
+// (1024 + 16 q) * (sc/16) - (64 + z) * sc = sc * (q - z), exact: `biased` holds 0x6400 | 16 q in both halves
+__device__ __forceinline__ uint32_t scale_codes(uint32_t biased, __half2 m, __half2 a) {
     const __half2 r = __hfma2(*reinterpret_cast<const __half2*>(&biased), m, a);
     return *reinterpret_cast<const uint32_t*>(&r);
+}
+
+
+// The scales of a row's super-block.  The drain applies s = d.  Where dmin is large beside d (blocks whose spread is small
+// beside their offset) the constant term would not fit a half: s = d * 2^k and the codes carry f = 2^-k, which halves hold
+// exactly up to k = 20.
+struct BlockScales {
+    uint32_t sc_lo, sc_hi, mn_lo, mn_hi;
+    float s = 0.f, f, rho;
+    bool any_wide;
+    template <bool Q5>
+    __device__ __forceinline__ void load(const uint4& w) {
+        const BlockHeader h{w.x, w.y, w.z, w.w};
+        const float d = half_bits_to_float(h.w0), dmin = half_bits_to_float(h.w0 >> 16);
+        unpack_scales_packed(h, sc_lo, sc_hi, mn_lo, mn_hi);
+        s = d, f = 1.f, rho = dmin / d;
+        const bool wide = !(fabsf(dmin) < 16.f * fabsf(d));
+        any_wide = __any_sync(0xFFFFFFFFu, wide);
+        if (wide) {
+            if (d == 0.f) {
+                f = 0.f, s = dmin * 0.0625f, rho = 16.f;
+            } else {
+                const uint32_t e = (__float_as_uint(rho) >> 23) & 255u;  // at least 131
+                f = __uint_as_float((257u - e) << 23);                   // rho * f in [8, 16)
+                s = d * __uint_as_float((e - 3u) << 23);
+                rho *= f;
+            }
+        }
+    }
+};
+// A 64-weight group's two scales sc (even and odd sub-block) as the operands of scale_codes.
+struct GroupScales {
+    __half2 me, mo, ae, ao;
+    __device__ __forceinline__ GroupScales(const BlockScales& h, uint32_t g, float z) {
+        const uint32_t scw = (g >= 2u ? h.sc_hi : h.sc_lo) >> (16u * (g & 1u));
+        // sc/16 in both halves of a register: 0x6400 | sc is 1024 + sc
+        const uint32_t be = __byte_perm(scw, 0x64u, 0x4040), bo = __byte_perm(scw, 0x64u, 0x4141);
+        const __half2 k16 = __float2half2_rn(0.0625f), k64 = __float2half2_rn(-64.f);
+        me = __hfma2(*reinterpret_cast<const __half2*>(&be), k16, k64), mo = __hfma2(*reinterpret_cast<const __half2*>(&bo), k16, k64);
+        if (h.any_wide) me = __float2half2_rn(__low2float(me) * h.f), mo = __float2half2_rn(__low2float(mo) * h.f);
+        const __half2 kz = __float2half2_rn(-(64.f + z) * 16.f);
+        ae = __hmul2(me, kz), ao = __hmul2(mo, kz);
+    }
+};
+// Four code words (16 code bytes: 16 weights of the even and 16 of the odd sub-block of group g) -> 16 columns of the
+// operand: per word the even sub-block's weights 4i, 4i+2 | 4i+1, 4i+3, then the odd one's.
+template <bool Q5>
+__device__ __forceinline__ void dequant_words(const uint4& code, const uint4& fifth, uint32_t g, const GroupScales& gs, uint32_t* v) {
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint32_t w = i == 0 ? code.x : i == 1 ? code.y : i == 2 ? code.z : code.w;
+        // codes 16 q under the half 1024; Q5_K: with the fifth bit above them
+        uint32_t f0 = 0x64006400u, f1 = f0, f2 = f0, f3 = f0;
+        if constexpr (Q5) {
+            const uint32_t q = (i == 0 ? fifth.x : i == 1 ? fifth.y : i == 2 ? fifth.z : fifth.w) >> (2u * g);  // bits 0 and 1 of each byte
+            auto fifth_of = [](uint32_t b) {
+                uint32_t r;
+                asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(r) : "r"(b), "r"(0x01000100u), "r"(0x64006400u));
+                return r;
+            };
+            f0 = fifth_of(q << 8), f1 = fifth_of(q), f2 = fifth_of(q << 7), f3 = fifth_of(q >> 1);
+        }
+        v[4 * i] = scale_codes(codes_of(w << 4, f0), gs.me, gs.ae);
+        v[4 * i + 1] = scale_codes(codes_of(w >> 4, f1), gs.me, gs.ae);
+        v[4 * i + 2] = scale_codes(codes_of(w, f2), gs.mo, gs.ao);
+        v[4 * i + 3] = scale_codes(codes_of(w >> 8, f3), gs.mo, gs.ao);
+    }
+}
+// The constant terms 32 * (z*sc*f - rho*mn) of the eight sub-blocks: four words of high halves, four of low ones.
+template <bool Q5>
+__device__ __forceinline__ void constant_terms(const BlockScales& h, uint32_t (&cw)[8]) {
+    const float zf = 32.f * (Q5 ? 16.f : 8.f) * h.f, rf = -32.f * h.rho;
+    // byte b of w as a float: 2^23 + byte is one permute away
+    auto byte_f = [](uint32_t w, uint32_t b) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | b)) - 8388608.f; };
+#pragma unroll
+    for (uint32_t p = 0; p < 4; p++) {
+        const uint32_t sw = p < 2 ? h.sc_lo : h.sc_hi, mw = p < 2 ? h.mn_lo : h.mn_hi, b = 2u * (p & 1u);
+        const float ce = fmaf(rf, byte_f(mw, b), zf * byte_f(sw, b));
+        const float co = fmaf(rf, byte_f(mw, b + 1u), zf * byte_f(sw, b + 1u));
+        cw[p] = half2_bits(ce, co);
+        const float2 cf = __half22float2(*reinterpret_cast<const __half2*>(&cw[p]));
+        cw[4 + p] = half2_bits(ce - cf.x, co - cf.y);
+    }
 }
 
 __device__ __forceinline__ uint32_t unit_begin(uint32_t cta, uint32_t base, uint32_t extra) { return cta * base + min(cta, extra); }
@@ -252,7 +341,9 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
     auto acc_full = [&](uint32_t rt, uint32_t b) { return bar0 + (C0 + (P::RB == 2u ? rt * 2u : 0u) + b) * 8u; };
     auto acc_empty = [&](uint32_t rt, uint32_t b) { return bar0 + (C0 + 4u + (P::RB == 2u ? rt * 2u : 0u) + b) * 8u; };
     const uint32_t done_bar = bar0 + (C0 + 8u) * 8u;
-    static_assert((C0 + 9u) * 8u + 16u <= P::BAR_BYTES, "barrier area");
+    auto s_full = [&](uint32_t rt, uint32_t s) { return bar0 + (C0 + 11u + rt * 4u + s) * 8u; };  // (after done_bar and 16 bytes of flags)
+    const uint32_t skew_bar = bar0 + (C0 + 19u) * 8u;
+    static_assert((C0 + 20u) * 8u <= P::BAR_BYTES, "barrier area");
     volatile int* abort_flag = reinterpret_cast<volatile int*>(base_ptr + OFF_BAR + (C0 + 9u) * 8u);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base_ptr + OFF_BAR + (C0 + 9u) * 8u + 4u);
     volatile uint32_t* last_flag = reinterpret_cast<volatile uint32_t*>(base_ptr + OFF_BAR + (C0 + 9u) * 8u + 8u);
@@ -262,13 +353,17 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
     const uint32_t nu = u1 - u0;
 
     if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < P::NR; s++) mbar_init(raw_full(s), 1), mbar_init(raw_empty(s), kWorkers / 2u);
-        for (uint32_t s = 0; s < P::NB; s++) mbar_init(b_full(s), 1), mbar_init(b_empty(s), 1);
+        for (uint32_t s = 0; s < P::NR; s++) mbar_init(raw_full(s), 1), mbar_init(raw_empty(s), P::WIDE ? 4u : 8u);
+        for (uint32_t s = 0; s < P::NB; s++) mbar_init(b_full(s), 1), mbar_init(b_empty(s), P::WIDE ? 2u : 1u);
         for (uint32_t rt = 0; rt < P::RB; rt++) {  // a group is dequantised by one of two sets of four warps per row tile
-            for (uint32_t s = 0; s < P::NA; s++) mbar_init(a_full(rt, s), 8u / P::RB), mbar_init(a_empty(rt, s), 1);
-            for (uint32_t b = 0; b < P::NBUF; b++) mbar_init(acc_full(rt, b), 1), mbar_init(acc_empty(rt, b), kWorkers / P::RB);
+            for (uint32_t s = 0; s < P::NA; s++) mbar_init(a_full(rt, s), P::WIDE ? 4u : 8u), mbar_init(a_empty(rt, s), 1);
+            for (uint32_t b = 0; b < P::NBUF; b++) mbar_init(acc_full(rt, b), 1), mbar_init(acc_empty(rt, b), P::WIDE ? 4u : 16u);
         }
-        mbar_init(done_bar, 1);
+        mbar_init(done_bar, P::WIDE ? 2u : 1u);
+        if constexpr (P::WIDE) {
+            for (uint32_t i = 0; i < 8; i++) mbar_init(s_full(i >> 2, i & 3u), 4);
+            mbar_init(skew_bar, 1);
+        }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -284,9 +379,9 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
     auto acc_col = [&](uint32_t rt, uint32_t b) { return (rt * P::NBUF + b) * P::N; };
     auto a_col = [&](uint32_t rt, uint32_t s) { return P::ACC_COLS + (rt * P::NA + s) * kASlotCols; };
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    // T > 64: 20 warps are launched with 96 registers a thread (61,440 in all); 16 x 112 + 4 x 32 is the same sum
+    // WIDE: 20 warps are launched with 96 registers a thread, 61,440 in all; 8 x 32 x (64 + 160) + 4 x 32 x 32 is the same sum
     if (warp < 4) {
-    if constexpr (T > 64) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    if constexpr (P::WIDE) asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
     if (warp == 0) {
         // ---------------- raw super-blocks ----------------
         if (lane == 0) {
@@ -332,7 +427,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
             if (!ok)
                 for (uint32_t i = issued > P::NB ? issued - P::NB : 0u; i < issued; i++) wait_in_flight(b_full(i % P::NB), (i / P::NB) & 1u);
         }
-    } else if (warp == 1) {
+    } else if (warp == 1 || P::WIDE) {
         // ---------------- mma issue ----------------
         // The whole warp walks the loop, one lane issues.  (With the loop under `lane == 0` every descriptor of every mma
         // was moved to uniform registers by itself: 110 cycles an mma, 5,100 cycles for the 34 small mmas of a unit.)
@@ -376,29 +471,26 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     if (++sb == P::NB) sb = 0, itb++;
                 }
             } else {
-                // position of each row tile: group i = 4*super-block + g, its slot in the two rings and how often the first has wrapped
-                uint32_t sb[2] = {0, 0}, itb = 0, sa[2] = {0, 0}, ita[2] = {0, 0};
-                const uint32_t ng = nu * 4u;
-                for (uint32_t j = 0; j < ng + P::LAG && ok; j++) {
+                // one issuing warp per row tile: while one waits for its accumulator to be drained the other keeps the tensor
+                // core busy (one warp for both stood still in every drain: 11,300 cycles a unit at T = 128, 4,300 of them mmas)
+                const uint32_t rt = warp >> 1;
+                uint32_t sb = 0, itb = 0, sa = 0, ita = 0;
+                if (rt == 1u) ok = wait_bar(skew_bar, 0, abort_flag, a.status);  // two groups behind: the drains alternate
+                for (uint32_t k = 0; k < nu && ok; k++) {
+                    if (k > 0) ok = wait_bar(acc_empty(rt, 0), (k - 1u) & 1u, abort_flag, a.status);
 #pragma unroll
-                    for (uint32_t rt = 0; rt < 2; rt++) {
-                        const uint32_t i = rt == 0 ? j : j - P::LAG;
-                        if (i >= ng) continue;  // (i wraps below zero while the second row tile has not started)
-                        const uint32_t g = i & 3u, k = i >> 2;
-                        if (rt == 0) ok &= wait_bar(b_full(sb[0]), itb & 1u, abort_flag, a.status);
-                        if (g == 0 && k > 0) ok &= wait_bar(acc_empty(rt, 0), (k - 1u) & 1u, abort_flag, a.status);
-                        ok &= wait_bar(a_full(rt, sa[rt]), ita[rt] & 1u, abort_flag, a.status);
+                    for (uint32_t g = 0; g < 4; g++) {
+                        ok &= wait_bar(b_full(sb), itb & 1u, abort_flag, a.status);
+                        ok &= wait_bar(a_full(rt, sa), ita & 1u, abort_flag, a.status);
                         fence_after();
-                        const uint32_t bt = b_slot(sb[rt]);
-                        group(tmem + acc_col(rt, 0), tmem + a_col(rt, sa[rt]), bt, bt + P::G_BYTES, g);
-                        umma_commit(leader, a_empty(rt, sa[rt]));
+                        const uint32_t bt = b_slot(sb);
+                        group(tmem + acc_col(rt, 0), tmem + a_col(rt, sa), bt, bt + P::G_BYTES, g);
+                        umma_commit(leader, a_empty(rt, sa));
+                        umma_commit(leader, b_empty(sb));
+                        if (g == 1 && k == 0 && rt == 0u) umma_commit(leader, skew_bar);
                         if (g == 3) umma_commit(leader, acc_full(rt, 0));
-                        if (rt == 1) umma_commit(leader, b_empty(sb[rt]));
-                        if (++sb[rt] == P::NB) {
-                            sb[rt] = 0;
-                            if (rt == 0) itb++;
-                        }
-                        if (++sa[rt] == P::NA) sa[rt] = 0, ita[rt]++;
+                        if (++sb == P::NB) sb = 0, itb++;
+                        if (++sa == P::NA) sa = 0, ita++;
                     }
                 }
             }
@@ -406,16 +498,130 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
             wait_in_flight(done_bar, 0);
         }
     }
+    } else if constexpr (P::WIDE) {
+        const uint32_t rt = ((warp - 4u) >> 2) & 1u, quad = warp & 3u;
+        const uint32_t row = quad * 32u + lane;            // lane of the row tile
+        const uint32_t tl = tmem + ((quad * 32u) << 16);   // this warp's lanes
+        float* s_ring = reinterpret_cast<float*>(base_ptr + OFF_BAR + P::BAR_BYTES) + rt * 128u + row;  // [super-block & 3][256]
+        if (warp < 12u) {
+            // ---------------- dequantise: one weight row per thread ----------------
+            asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+            uint32_t rs = rt, rit = 0, sa = 0, ita = 0;
+            for (uint32_t k = 0; k < nu; k++) {
+                wait_bar(raw_full(rs), rit & 1u, abort_flag, a.status);
+                const uint32_t rp = raw_slot(rs) + row * P::BLOCK;
+                BlockScales h;
+                h.load<Q5>(lds128(rp));
+                // (read four super-blocks from now at the earliest: the operand ring is shorter than one)
+                s_ring[(k & 3u) * 256u] = h.s;
+                __syncwarp();
+                if (lane == 0) mbar_arrive(s_full(rt, k & 3u));
+#pragma unroll
+                for (uint32_t g = 0; g < 4; g++) {
+                    const GroupScales gs(h, g, Q5 ? 16.f : 8.f);
+                    const uint32_t ta = tl + a_col(rt, sa);
+                    if (ita > 0) wait_bar(a_empty(rt, sa), (ita - 1u) & 1u, abort_flag, a.status);
+                    __syncwarp();
+                    fence_after();
+#pragma unroll
+                    for (uint32_t hf = 0; hf < 2; hf++) {
+                        uint32_t v[16];
+                        const uint4 code = lds128(rp + (Q5 ? 48u : 16u) + g * 32u + hf * 16u);
+                        uint4 fifth = make_uint4(0, 0, 0, 0);
+                        if constexpr (Q5) fifth = lds128(rp + 16u + hf * 16u);
+                        dequant_words<Q5>(code, fifth, g, gs, v);
+                        tmem_st16(ta + hf * 16u, v);
+                    }
+                    if (g == 3) {
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(raw_empty(rs));
+                        rs += 2u;
+                        if (rs >= P::NR) rs -= P::NR, rit++;
+                        uint32_t cw[8];
+                        constant_terms<Q5>(h, cw);
+                        tmem_st8(ta + 32u, cw);
+                    }
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(a_full(rt, sa));
+                    if (++sa == P::NA) sa = 0, ita++;
+                }
+            }
+        } else {
+            // ---------------- drain: the T partial sums of one weight row per thread ----------------
+            asm volatile("setmaxnreg.inc.sync.aligned.u32 160;");
+            float y[T];
+#pragma unroll
+            for (int j = 0; j < T; j++) y[j] = 0.f;
+            uint32_t tile = u0 / a.nsb, b = u0 - tile * a.nsb;
+            bool seg_head = b == 0;
+            for (uint32_t k = 0; k < nu; k++) {
+                wait_bar(s_full(rt, k & 3u), (k >> 2) & 1u, abort_flag, a.status);
+                const float sc = s_ring[(k & 3u) * 256u];
+                wait_bar(acc_full(rt, 0), k & 1u, abort_flag, a.status);
+                __syncwarp();
+                fence_after();
+                const uint32_t col = tl + acc_col(rt, 0);
+#pragma unroll
+                for (int c0 = 0; c0 < T; c0 += 16) {
+                    uint32_t v[16];
+                    tmem_ld<16>(col + c0, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c0 + 16 == T) {
+                        fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(acc_empty(rt, 0));
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; j++) {
+                        y[c0 + j] = fmaf(sc, __uint_as_float(v[j]), y[c0 + j]);
+                        asm volatile("" : "+f"(y[c0 + j]));  // (before the next load: else all T loaded values wait in registers)
+                    }
+                }
+                const bool tile_end = b + 1u == a.nsb;
+                if (tile_end || k + 1u == nu) {
+                    // a whole tile goes to Y, a cut one to the workspace
+                    asm volatile("griddepcontrol.wait;" ::: "memory");
+                    const uint32_t rtile = tile / a.tok_tiles, tok0 = (tile - rtile * a.tok_tiles) * T;
+                    const uint32_t n = rtile * kTileRows + rt * 128u + row, tok_n = min(a.M - tok0, (uint32_t)T);
+                    const bool whole = tile_end && seg_head;
+                    float* out = whole ? a.Y + (uint64_t)tok0 * a.N + n
+                                       : a.part + ((uint64_t)blockIdx.x * 2u + (seg_head ? 1u : 0u)) * a.slot_rows * kTileRows + rt * 128u + row;
+                    const uint32_t stride = whole ? a.N : kTileRows;
+                    const float bias = whole && a.bias && n < a.N ? a.bias[n] : 0.f;
+                    const bool row_ok = n < a.N || !whole;
+                    // 2^-e of 32 activation rows a turn, one per lane: a load per value would cost the turn an L2 latency each
+                    float iv = whole && lane < tok_n ? __ldcg(a.inv + tok0 + lane) : 1.f;
+                    // 32 columns a turn, the rest moved down: the loop keeps the compiler from holding every column's address
+                    // beside the sums (it spilled 114 of the 128), and leaves zeros behind
+#pragma unroll 1
+                    for (uint32_t c0 = 0; c0 < (uint32_t)T; c0 += 32) {
+                        const float ivn = whole && c0 + 32u + lane < tok_n ? __ldcg(a.inv + tok0 + c0 + 32u + lane) : 1.f;
+#pragma unroll
+                        for (uint32_t j = 0; j < 32; j++) {
+                            const float r = fmaf(y[j], __shfl_sync(0xFFFFFFFFu, iv, j), bias);
+                            if (c0 + j < tok_n && row_ok) *out = r;
+                            out += stride;
+                        }
+                        iv = ivn;
+#pragma unroll
+                        for (int j = 0; j < T; j++) y[j] = j + 32 < T ? y[j + 32 < T ? j + 32 : j] : 0.f;
+                    }
+                    seg_head = true;
+                }
+                if (tile_end) b = 0, tile++;
+                else b++;
+            }
+            fence_before();
+        }
     } else {
         // ---------------- dequantise, drain ----------------
-        if constexpr (T > 64) asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
         const uint32_t wk = warp - 4u, rt = wk >> 3, set = (wk >> 2) & 1u, quad = warp & 3u;
         const uint32_t row = quad * 32u + lane;            // lane of the row tile
         const uint32_t tl = tmem + ((quad * 32u) << 16);   // this warp's lanes
         constexpr int TH = T / 2;                          // columns this warp drains: [set*TH, set*TH + TH)
         constexpr int CH = TH % 16 == 0 ? 16 : TH % 8 == 0 ? 8 : 4;
-        constexpr float Z = Q5 ? 16.f : 8.f;
-        constexpr uint32_t CU = Q5 ? 48u : 16u;            // first code byte of a block
         float y[TH];
 #pragma unroll
         for (int j = 0; j < TH; j++) y[j] = 0.f;
@@ -431,28 +637,22 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
             __syncwarp();
             fence_after();
             const uint32_t col = tl + acc_col(rt, buf) + set * TH;
-            constexpr int STEP = TH <= 32 ? TH : TH % 16 == 0 ? 16 : 8;  // columns in registers at a time beside the sums
+            uint32_t hi[TH];
+            [[maybe_unused]] uint32_t lo[P::STACK ? TH : 1];
 #pragma unroll
-            for (int c0 = 0; c0 < TH; c0 += STEP) {
-                uint32_t hi[STEP];
-                [[maybe_unused]] uint32_t lo[P::STACK ? STEP : 1];
+            for (int c = 0; c < TH; c += CH) {
+                tmem_ld<CH>(col + c, hi + c);
+                if constexpr (P::STACK) tmem_ld<CH>(col + T + c, lo + c);
+            }
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(acc_empty(rt, buf));
 #pragma unroll
-                for (int c = 0; c < STEP; c += CH) {
-                    tmem_ld<CH>(col + c0 + c, hi + c);
-                    if constexpr (P::STACK) tmem_ld<CH>(col + T + c0 + c, lo + c);
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c0 + STEP == TH) {
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(acc_empty(rt, buf));
-                }
-#pragma unroll
-                for (int j = 0; j < STEP; j++) {
-                    float v = __uint_as_float(hi[j]);
-                    if constexpr (P::STACK) v += __uint_as_float(lo[j]);
-                    y[c0 + j] = fmaf(s_prev, v, y[c0 + j]);
-                }
+            for (int j = 0; j < TH; j++) {
+                float v = __uint_as_float(hi[j]);
+                if constexpr (P::STACK) v += __uint_as_float(lo[j]);
+                y[j] = fmaf(s_prev, v, y[j]);
             }
             const bool tile_end = db + 1u == a.nsb;
             if (tile_end || kd + 1u == nu) {
@@ -486,7 +686,6 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 #pragma unroll
                             for (int j = 0; j < TH; j++) {
                                 if (t0 + j < tok_n) y[j] += __ldcg(p + j * kTileRows);
-                                if (TH > 32 && j % 16 == 15) asm volatile("" ::: "memory");  // (registers)
                             }
                         }
                     }
@@ -514,125 +713,49 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 
         for (uint32_t k = 0; k <= nu; k++) {
             const bool more = k < nu;
-            float s_cur = 0.f, f = 1.f, d = 0.f, dmin = 0.f, rho = 0.f;
-            uint32_t sc_lo = 0, sc_hi = 0, mn_lo = 0, mn_hi = 0;
-            const uint32_t rp = raw_slot(rs) + row * P::BLOCK;
-            bool wide = false, any_wide = false;
+            BlockScales h;
             if (more) {
-            wait_bar(raw_full(rs), rit & 1u, abort_flag, a.status);
-            const uint4 h4 = lds128(rp);
-            const BlockHeader h{h4.x, h4.y, h4.z, h4.w};
-            d = half_bits_to_float(h.w0), dmin = half_bits_to_float(h.w0 >> 16);
-            unpack_scales_packed(h, sc_lo, sc_hi, mn_lo, mn_hi);
-            // The drain applies s = d.  Where dmin is large beside d (blocks whose spread is small beside their offset) the
-            // constant term would not fit a half: s = d * 2^k and the codes carry 2^-k, which halves hold exactly up to k = 20.
-            s_cur = d;
-            wide = !(fabsf(dmin) < 16.f * fabsf(d));
-            if (wide) {
-                if (d == 0.f) {
-                    f = 0.f, s_cur = dmin * 0.0625f, rho = 16.f;
-                } else {
-                    const float r = dmin / d;
-                    const uint32_t e = (__float_as_uint(r) >> 23) & 255u;  // at least 131
-                    f = __uint_as_float((257u - e) << 23);                 // r * f in [8, 16)
-                    s_cur = d * __uint_as_float((e - 3u) << 23);
-                    rho = r * f;
-                }
-            }
-            any_wide = __any_sync(0xFFFFFFFFu, wide);
-            }
+                wait_bar(raw_full(rs), rit & 1u, abort_flag, a.status);
+                const uint32_t rp = raw_slot(rs) + row * P::BLOCK;
+                h.load<Q5>(lds128(rp));
 #pragma unroll
-            for (uint32_t gi = 0; gi < 2; gi++) {
-                if (more) {
-                // 64-weight group g = set + 2*gi: sub-blocks 2g and 2g+1
-                const uint32_t cp = rp + CU + (set + 2u * gi) * 32u;
-                const uint32_t scw = (gi ? sc_hi : sc_lo) >> (16u * set);
-                // sc/16 in both halves of a register: 0x6400 | sc is 1024 + sc
-                const uint32_t be = __byte_perm(scw, 0x64u, 0x4040), bo = __byte_perm(scw, 0x64u, 0x4141);
-                const __half2 k16 = __float2half2_rn(0.0625f), k64 = __float2half2_rn(-64.f);
-                __half2 me = __hfma2(*reinterpret_cast<const __half2*>(&be), k16, k64), mo = __hfma2(*reinterpret_cast<const __half2*>(&bo), k16, k64);
-                if (any_wide) me = __float2half2_rn(__low2float(me) * f), mo = __float2half2_rn(__low2float(mo) * f);
-                const __half2 kz = __float2half2_rn(-(64.f + Z) * 16.f);
-                const __half2 ae = __hmul2(me, kz), ao = __hmul2(mo, kz);
-                const uint32_t ta = tl + a_col(rt, sa);
-                auto release_raw = [&] {
+                for (uint32_t gi = 0; gi < 2; gi++) {
+                    const uint32_t g = set + 2u * gi;  // 64-weight group: sub-blocks 2g and 2g+1
+                    const uint32_t cp = rp + (Q5 ? 48u : 16u) + g * 32u;
+                    const GroupScales gs(h, g, Q5 ? 16.f : 8.f);
+                    const uint32_t ta = tl + a_col(rt, sa);
+                    const uint4 code[2] = {lds128(cp), lds128(cp + 16u)};
+                    uint4 fifth[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+                    if constexpr (Q5) fifth[0] = lds128(rp + 16u), fifth[1] = lds128(rp + 32u);
                     if (gi == 1) {
                         __syncwarp();
                         if (lane == 0) mbar_arrive(raw_empty(rs));
                         rs += 2u;
                         if (rs >= P::NR) rs -= P::NR, rit++;
                     }
-                };
-                auto wait_slot = [&] {
+                    uint32_t v[32];
+                    dequant_words<Q5>(code[0], fifth[0], g, gs, v);
+                    dequant_words<Q5>(code[1], fifth[1], g, gs, v + 16);
                     if (ita > 0) wait_bar(a_empty(rt, sa), (ita - 1u) & 1u, abort_flag, a.status);
                     __syncwarp();
                     fence_after();
-                };
-                constexpr bool WHOLE = TH <= 32;  // (registers: else a half group at a time)
-                if constexpr (!WHOLE) wait_slot();
-                constexpr int VW = WHOLE ? 32 : 16;
-#pragma unroll
-                for (int hf = 0; hf < 32; hf += VW) {
-                    uint4 code[VW / 16];
-                    [[maybe_unused]] uint4 fifth[VW / 16];
-#pragma unroll
-                    for (int q = 0; q < VW / 16; q++) {
-                        code[q] = lds128(cp + hf + q * 16u);
-                        if constexpr (Q5) fifth[q] = lds128(rp + 16u + hf + q * 16u);
+                    tmem_st16(ta, v);
+                    tmem_st16(ta + 16u, v + 16);
+                    if (gi == 1 && set == 1) {  // the last group of the super-block carries the constant terms of its eight sub-blocks
+                        uint32_t cw[8];
+                        constant_terms<Q5>(h, cw);
+                        tmem_st8(ta + 32u, cw);
                     }
-                    if (hf + VW == 32) release_raw();
-                    uint32_t v[VW];
-#pragma unroll
-                    for (int iv = 0; iv < VW / 4; iv++) {
-                        const uint4 cu = code[iv >> 2];
-                        const uint32_t w = (iv & 3) == 0 ? cu.x : (iv & 3) == 1 ? cu.y : (iv & 3) == 2 ? cu.z : cu.w;
-                        uint32_t p0 = (w << 4) & 0x00F000F0u, p1 = (w >> 4) & 0x00F000F0u;  // even sub-block: weights 4i, 4i+2 | 4i+1, 4i+3
-                        uint32_t p2 = w & 0x00F000F0u, p3 = (w >> 8) & 0x00F000F0u;         // odd sub-block
-                        if constexpr (Q5) {
-                            const uint4 fu = fifth[iv >> 2];
-                            const uint32_t fw = (iv & 3) == 0 ? fu.x : (iv & 3) == 1 ? fu.y : (iv & 3) == 2 ? fu.z : fu.w;
-                            const uint32_t q = fw >> (2u * set + 4u * gi);  // bits 0 and 1 of each byte: even, odd sub-block
-                            p0 |= (q << 8) & 0x01000100u;
-                            p1 |= q & 0x01000100u;
-                            p2 |= (q << 7) & 0x01000100u;
-                            p3 |= (q >> 1) & 0x01000100u;
-                        }
-                        v[4 * iv] = scale_codes(p0, me, ae);
-                        v[4 * iv + 1] = scale_codes(p1, me, ae);
-                        v[4 * iv + 2] = scale_codes(p2, mo, ao);
-                        v[4 * iv + 3] = scale_codes(p3, mo, ao);
-                    }
-                    if constexpr (WHOLE) wait_slot();
-#pragma unroll
-                    for (int q = 0; q < VW; q += 16) tmem_st16(ta + hf + q, v + q);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(a_full(rt, sa));
+                    sa += 2u;
+                    if (sa >= P::NA) sa -= P::NA, ita++;
                 }
-                if (gi == 1 && set == 1) {  // the last group of the super-block carries the constant terms of its eight sub-blocks
-                    if (!wide) rho = dmin / d;
-                    const float zf = 32.f * Z * f, rf = -32.f * rho;
-                    // byte b of w as a float: 2^23 + byte is one permute away
-                    auto byte_f = [](uint32_t w, uint32_t b) { return __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u | b)) - 8388608.f; };
-                    uint32_t cw[8];
-#pragma unroll
-                    for (uint32_t p = 0; p < 4; p++) {
-                        const uint32_t sw = p < 2 ? sc_lo : sc_hi, mw = p < 2 ? mn_lo : mn_hi, b = 2u * (p & 1u);
-                        const float ce = fmaf(rf, byte_f(mw, b), zf * byte_f(sw, b));
-                        const float co = fmaf(rf, byte_f(mw, b + 1u), zf * byte_f(sw, b + 1u));
-                        cw[p] = half2_bits(ce, co);
-                        const float2 cf = __half22float2(*reinterpret_cast<const __half2*>(&cw[p]));
-                        cw[4 + p] = half2_bits(ce - cf.x, co - cf.y);
-                    }
-                    tmem_st8(ta + 32u, cw);
-                }
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(a_full(rt, sa));
-                sa += 2u;
-                if (sa >= P::NA) sa -= P::NA, ita++;
-                }
-                if (gi == (P::NBUF == 1u ? 0u : 1u) && k > 0) drain(k - 1u);
             }
-            s_prev = s_cur;
+            if (k > 0) drain(k - 1u);
+            s_prev = h.s;
         }
         fence_before();
     }
@@ -719,17 +842,18 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
 // Cut tiles: the sum of the segments in ascending order of k, times 2^-e, plus the bias.  Where tiles are cut into many
 // segments one CTA would add them with a chain of L2 latencies (1024 x 4096, 48 rows: 16 segments, 50 of 77 us); here
 // a thread takes four weight rows of one activation row and the whole machine shares the work.
-// One block: one tile, four activation rows.
+// One block: the tile that CTA blockIdx.x begins and others finish, four activation rows.
 __global__ void __launch_bounds__(256) rows_reduce_kernel(const float* __restrict__ part, const float* __restrict__ inv,
                                                           const float* __restrict__ bias, float* __restrict__ Y, uint32_t M, uint32_t N,
                                                           uint32_t T, uint32_t tok_tiles, uint32_t slot_rows, uint32_t nsb, uint32_t u_base,
                                                           uint32_t u_extra) {
-    const uint32_t tile = blockIdx.x, rtile = tile / tok_tiles, tok0 = (tile - rtile * tok_tiles) * T;
+    const uint32_t tile = (unit_begin(blockIdx.x + 1u, u_base, u_extra) - 1u) / nsb;
+    const uint32_t rtile = tile / tok_tiles, tok0 = (tile - rtile * tok_tiles) * T;
     const uint32_t t = blockIdx.y * 4u + (threadIdx.x >> 6), r4 = (threadIdx.x & 63u) * 4u, n = rtile * kTileRows + r4;
     const uint32_t c_first = unit_owner(tile * nsb, u_base, u_extra), c_last = unit_owner((tile + 1u) * nsb - 1u, u_base, u_extra);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (c_first == c_last || t >= slot_rows || tok0 + t >= M || n >= N) return;
+    if (c_first != blockIdx.x || c_first == c_last || t >= slot_rows || tok0 + t >= M || n >= N) return;
     const uint64_t slot = (uint64_t)slot_rows * kTileRows;
     const float* p = part + (uint64_t)c_first * 2u * slot + t * kTileRows + r4;
     float4 s = __ldcg(reinterpret_cast<const float4*>(p + slot));
@@ -849,7 +973,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, uint32_t* counters, void* buffer
     ra.u_base = units / grid;
     ra.u_extra = units % grid;
     // a tile of nsb units is cut into at most (nsb - 2) / u_base + 2 segments; up to three the last CTA adds them itself
-    ra.defer = nsb > 1u && (nsb - 2u) / ra.u_base + 2u > 3u;
+    ra.defer = T > 48u ? 1u : nsb > 1u && (nsb - 2u) / ra.u_base + 2u > 3u;
     const uint32_t key_nb = nsb | (q5 ? 0x50000000u : 0u), key_cb = 0x80u;  // apart from the streaming kernel's boxes of the same weights
     bool found = false;
     if (tmaps)
@@ -893,7 +1017,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, uint32_t* counters, void* buffer
     e = q5 ? launch_rows_t<1>(T, ra, grid, pdl, stream) : launch_rows_t<0>(T, ra, grid, pdl, stream);
     if (launches) ++*launches;
     if (e != cudaSuccess || !ra.defer) return e;
-    cfg.gridDim = dim3(((m.N + kTileRows - 1u) / kTileRows) * tok_tiles, (ra.slot_rows + 3u) / 4u);
+    cfg.gridDim = dim3(grid, (ra.slot_rows + 3u) / 4u);
     e = cudaLaunchKernelEx(&cfg, rows_reduce_kernel, (const float*)ra.part, ra.inv, ra.bias, ra.Y, ra.M, ra.N, T, tok_tiles, ra.slot_rows, nsb,
                            ra.u_base, ra.u_extra);
     if (launches) ++*launches;

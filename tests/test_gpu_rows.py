@@ -44,7 +44,9 @@ def close(y, x, w64, bias=None):
 
 # every activation tile (8 .. 64), ragged rows of weights, one block to many, cut and whole tiles
 SHAPES = [(5, 1, 256), (8, 300, 1024), (9, 256, 512), (16, 4099, 1024), (17, 511, 768), (24, 1000, 2560), (25, 257, 4096),
-          (32, 640, 256), (33, 513, 1024), (48, 300, 1792), (49, 700, 1280), (64, 130, 4096), (64, 40000, 1024), (40, 300, 512)]
+          (32, 640, 256), (33, 513, 1024), (48, 300, 1792), (49, 700, 1280), (64, 130, 4096), (64, 40000, 1024), (40, 300, 512), (65, 255, 1024),
+          (80, 512, 1024), (96, 300, 2048), (97, 1030, 1280), (112, 200, 1280), (128, 777, 1024), (129, 300, 1024), (200, 600, 1024),
+          (300, 520, 1024), (513, 260, 2048), (384, 9000, 1024)]
 
 
 @pytest.mark.parametrize("qtype", [q4k.Q4_K, q4k.Q5_K], ids=["q4_k", "q5_k"])
@@ -66,7 +68,7 @@ def test_rows_kernel_matches_64_bits(ctx, qtype, M, N, K):
     assert torch.equal(y, y2)                 # cut tiles are summed in a fixed order
 
 
-@pytest.mark.parametrize("M", [7, 20, 40, 64])
+@pytest.mark.parametrize("M", [7, 20, 40, 64, 90])
 def test_rows_kernel_range_of_activations_and_scales(ctx, M):
     """Rows from 1e-30 to 1e30 in magnitude, a zero row, one outlier beside small values; super-blocks whose d is zero, or
     tiny beside dmin, and blocks without a minimum."""
