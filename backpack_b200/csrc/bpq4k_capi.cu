@@ -22,7 +22,7 @@ struct bpq4k_context {
     int prefill_variant = 0;  // BPQ4K_OPT_PREFILL_VARIANT
     int prefill_arg() const { return prefill_mode | (prefill_variant << 4); }  // what the launcher takes
     int prefill_min_m = 25;  // four 8-row slabs of the streaming kernel cost as much as one tensor-core pass
-    int rows_min_m = 9;  // smallest M of the several-rows kernel (takes_rows_kernel)
+    int rows_min_m = 0;  // 0: automatic; smallest M of the several-rows kernel (takes_rows_kernel)
     // its workspaces, one per stream that uses it (overlapping calls on two streams must not share one): counters and
     // the buffer of calls of up to kRowsFixedM rows; two are allocated with the handle (a program's stream and the one it
     // captures graphs on), two more when needed
@@ -193,14 +193,17 @@ uint8_t* rows_workspace(bpq4k_context* h, cudaStream_t st) {
     return nullptr;
 }
 
-// Which Q4_K / Q5_K calls take the several-rows kernel.  Below rows_min_m (9) the streaming kernel is as fast: it reads
-// the weights once for 8 rows (128256 x 4096: 8 rows 101 us against 105 here, 9 rows 150 against 105); below prefill_min_m it stops at 24 rows (a caller who moves the tensor-core threshold up asks for the streaming
+// Which Q4_K / Q5_K calls take the several-rows kernel.  To 8 rows the streaming kernel reads the
+// weights once too and is as fast while their digits fit in shared memory (8 rows, 6144 x 4096 13.3 us against 13.5 here,
+// 128256 x 4096 101 | 97; 9 rows 150 | 97); from K = 8192 on 5 rows do not (5 rows, 57344 x 8192 109 | 88, 8192 x 28672
+// 70 | 50, 4096 x 8192 17 | 16; 4 rows 74 | 88 and 49 | 50).  Below prefill_min_m it stops at 24 rows (a caller who moves the tensor-core threshold up asks for the streaming
 // kernel); at and above the threshold it keeps the float accuracy of the F16X3 mode, so the 16-bit modes, which ask for
 // less, stay with their own kernel.  More than 32 rows of a short K stay with the prefill kernel: from 33 rows on high and
 // low halves share an accumulator, 5.7e-7 of error at any K; the prefill kernel has 3.5e-7 at K = 256, 1.2e-6 at K = 1024.
 bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a, int qtype) {
     if (h->gemv_variant != BPQ4K_GEMV_AUTO || a.n_slots || a.n_peers || !aligned16(a.X)) return false;
-    if (a.M < (uint32_t)h->rows_min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u)) return false;
+    const uint32_t min_m = h->rows_min_m ? (uint32_t)h->rows_min_m : a.K >= 8192u ? 5u : 9u;
+    if (a.M < min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u)) return false;
     if (a.M < (uint32_t)h->prefill_min_m) return a.M <= 24u;
     if (h->prefill_mode != BPQ4K_PREFILL_F16X3) return false;
     // Against the prefill kernel (us, prefill | here).  To 96 rows here: 80 rows, 6144 x 4096 33 | 26, 128256 x 4096 350 | 195.
@@ -403,7 +406,7 @@ int bpq4k_set_option(bpq4k_handle_t h, int option, int value) {
             h->prefill_min_m = value;
             return BPQ4K_OK;
         case BPQ4K_OPT_ROWS_MIN_M:
-            if (value < 1) return fail(h, BPQ4K_ERR_INVALID_ARG, "rows_min_m must be >= 1");
+            if (value < 0) return fail(h, BPQ4K_ERR_INVALID_ARG, "rows_min_m must be >= 0");
             h->rows_min_m = value;
             return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_WARPS:

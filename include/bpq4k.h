@@ -116,7 +116,8 @@ typedef enum bpq4k_option {
      * BPQ4K_ERR_INVALID_ARG (even untaken, the six branches cost its decode step 2 %).  No counterpart in the reference. */
     BPQ4K_OPT_STREAM_STAMPS = 24,
     /* Smallest M of Q4_K and Q5_K matmuls that the several-rows kernel serves (K <= 32768).  From BPQ4K_OPT_PREFILL_MIN_M
-     * on it serves the F16X3 mode, below it M <= 24.  Default 9. */
+     * on it serves the F16X3 mode, below it M <= 24.  Default 0: automatic
+     * (9; 5 from K = 8192 on). */
     BPQ4K_OPT_ROWS_MIN_M = 25,
     /* Read-only (bpq4k_get_option): how many times bpq4k_matmul_host_batch_f32 has recorded a dispatch
      * list into a replay graph on this handle.  A list is recorded again after any of the handle's
