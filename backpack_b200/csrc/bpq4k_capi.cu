@@ -163,10 +163,8 @@ inline uint32_t stream_slab_rows(uint32_t K) { return (uint64_t)K * 16u * 4u <= 
 
 int alloc_rows_workspace(bpq4k_context::RowsWorkspace& w) {
     const size_t bytes = bpq4k_context::kRowsCounterBytes + rows_buffer_bytes(bpq4k_context::kRowsFixedM, kRowsMaxK);
-    if (cudaMalloc(reinterpret_cast<void**>(&w.mem), bytes) == cudaSuccess && cudaMemset(w.mem, 0, bpq4k_context::kRowsCounterBytes) == cudaSuccess)
-        return BPQ4K_OK;
+    if (cudaMalloc(reinterpret_cast<void**>(&w.mem), bytes) == cudaSuccess) return BPQ4K_OK;  // (each call clears its counters itself)
     cudaGetLastError();
-    if (w.mem) cudaFree(w.mem);
     w.mem = nullptr;
     return BPQ4K_ERR_ALLOC;
 }

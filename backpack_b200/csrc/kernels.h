@@ -149,8 +149,8 @@ size_t prefill_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int mode, int s
 cudaError_t launch_prefill_tc(const MatmulArgs& a, int mode, void* scratch, size_t scratch_bytes, int* status_dev,
                               int sm_count, cudaStream_t stream, int* launches, int qtype = 12);  // 12 Q4_K, 13 Q5_K, 0x10E padded Q6_K
 
-// Matmul of several activation rows, K up to 32768 (q4k_rows_tc.cu), two or three launches.  `counters`: 160 words that are zero
-// before the first call; `buffer`: rows_buffer_bytes() bytes; both serve one stream at a time.
+// Matmul of several activation rows, K up to 32768 (q4k_rows_tc.cu), two or three launches.  `counters`: 160 words,
+// `buffer`: rows_buffer_bytes() bytes; what they hold before a call does not matter, and both serve one call at a time.
 // cudaErrorInvalidValue: not a shape or form of this kernel.
 constexpr uint32_t kRowsMaxM = 16384, kRowsMaxK = 32768;
 size_t rows_buffer_bytes(uint32_t M, uint32_t K);

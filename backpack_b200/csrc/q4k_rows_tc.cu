@@ -47,6 +47,7 @@ namespace {
 
 constexpr uint32_t kWaitLimit = 1u << 21;
 constexpr uint32_t kSuspendNs = 1000;                 // a waiting warp sleeps this long at most: polls take issue slots from the dequantising warps
+constexpr uint32_t kMaxCtas = 160;                    // counters (one per CTA)
 constexpr uint32_t kWorkers = 16;                     // warps that dequantise and drain
 constexpr uint32_t kThreads = (4 + kWorkers) * 32;
 constexpr uint32_t kTileRows = 256;                   // weight rows of a unit: two row tiles of 128 lanes
@@ -96,7 +97,7 @@ struct RowsArgs {
     uint32_t tok_tiles, slot_rows;  // activation tiles; rows of a workspace slot (min(M, T))
     uint32_t defer;           // cut tiles are added up by rows_reduce_kernel
     float* part;              // [CTA][2][slot_rows][256]
-    uint32_t* counters;       // one per CTA, zero between launches
+    uint32_t* counters;       // one per CTA, cleared by rows_pack_kernel
     int* status;
 };
 
@@ -674,7 +675,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     const uint32_t c_last = unit_owner((dtile + 1u) * a.nsb - 1u, a.u_base, a.u_extra);
                     __threadfence();
                     asm volatile("bar.sync 1, %0;" ::"n"(kWorkers * 32) : "memory");
-                    if (threadIdx.x == 4u * 32u) *last_flag = atomicInc(a.counters + c_first, c_last - c_first);
+                    if (threadIdx.x == 4u * 32u) *last_flag = atomicAdd(a.counters + c_first, 1u);
                     asm volatile("bar.sync 1, %0;" ::"n"(kWorkers * 32) : "memory");
                     write = *last_flag == c_last - c_first;  // this CTA is the tile's last: add the segments in order of k
                     if (write) {
@@ -774,14 +775,18 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 // (both 16-byte chunks alike, so there is no swizzle to apply).
 // A block serves one row; where the rows alone do not fill the machine several blocks share one, and each finds the
 // row's maximum itself.  Rows past M are zeros.
+// The matmul's counters are cleared here, in the order of the call's own stream, so that no call depends on what the memory
+// held before it (a clear by another stream's memset would not be ordered against the kernel).
 __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict__ X, uint32_t M, uint32_t K, uint32_t T,
-                                                        uint8_t* __restrict__ image, float* __restrict__ inv) {
+                                                        uint8_t* __restrict__ image, float* __restrict__ inv,
+                                                        uint32_t* __restrict__ counters) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ uint32_t red[8];
     const uint32_t row = blockIdx.y, tt = row / T, t = row - tt * T, warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t nsb = K / kQK;
     const bool live = row < M;
+    if (row == 0 && blockIdx.x == 0 && threadIdx.x < kMaxCtas) counters[threadIdx.x] = 0;
     const float4* x4 = reinterpret_cast<const float4*>(X + (uint64_t)row * K);
     float scale = 0.f;
     if (live) {
@@ -891,8 +896,6 @@ uint32_t rows_tile(uint32_t M) {
     const uint32_t tiles = (M + 127u) / 128u, per = (M + tiles - 1u) / tiles;
     return per <= 32u ? (per + 7u) & ~7u : per <= 48u ? 48u : (per + 15u) & ~15u;
 }
-
-constexpr uint32_t kMaxCtas = 160;
 
 template <int T, int QT>
 cudaError_t launch_rows(const RowsArgs& ra, uint32_t grid, bool pdl, cudaStream_t stream) {
@@ -1011,7 +1014,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, uint32_t* counters, void* buffer
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv));
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv), counters);
     if (launches) ++*launches;
     if (e != cudaSuccess) return e;
     e = q5 ? launch_rows_t<1>(T, ra, grid, pdl, stream) : launch_rows_t<0>(T, ra, grid, pdl, stream);

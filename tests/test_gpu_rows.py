@@ -159,3 +159,42 @@ def test_rows_kernel_threshold_streams_and_capture(ctx):
         del g
     finally:
         c.close()
+
+
+def test_rows_kernel_first_call_of_a_stream_beside_a_busy_default_stream():
+    """The counters that elect the CTA which adds up a cut tile are cleared in the order of the calling stream: first calls
+    on side streams (non-blocking, as torch makes them) while the default stream is busy, on a handle whose default stream
+    has not been used.  600 units over 148 CTAs of whole shares of four: tiles are cut into two and the last CTA adds them
+    (no launch of its own for the sums)."""
+    import torch
+
+    import backpack_b200 as bp
+
+    M, N, K = 12, 38400, 1024
+    c = bp.Q4KContext(0)
+    try:
+        raw = synth.make_q4k_weights(N, K, 31)
+        w = c.upload(q4k.pack_q4k(raw, N, K))
+        xd = [torch.from_numpy(synth.make_activations(M, K, 40 + i)).cuda() for i in range(4)]
+        w64 = c.dequant(w).double()
+        want = [x.double() @ w64.T for x in xd]
+        del w64
+        ys = [torch.empty(M, N, device="cuda") for _ in xd]
+        streams = [torch.cuda.Stream() for _ in xd]
+        a = torch.randn(8192, 8192, device="cuda")
+        torch.cuda.synchronize()
+        c.launch_count(reset=True)
+        for _ in range(20):                   # tens of milliseconds of work on the default stream
+            torch.mm(a, a)
+        for x, y, s in zip(xd, ys, streams):
+            with torch.cuda.stream(s):
+                for _ in range(3):
+                    c.matmul(x, w, out=y)
+        torch.cuda.synchronize()
+        assert c.device_status() == 0
+        if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+            assert c.launch_count() == 2 * 3 * len(xd)
+        for y, v in zip(ys, want):
+            assert float((y.double() - v).norm() / v.norm()) <= 4e-6
+    finally:
+        c.close()
