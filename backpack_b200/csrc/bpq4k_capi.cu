@@ -5,11 +5,27 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <memory>
+#include <mutex>
 #include <new>
+#include <vector>
 
 #include "kernels.h"
 
 using namespace bpq4k;
+
+// Device blocks that captured calls use.  A graph that holds a call's kernels holds a reference on the call's block (a CUDA
+// user object): the block serves another capture only when the graph, every executable made or updated from it and every
+// launch in flight are gone.  Shared between the handle and the graphs, since a graph may outlive the handle.
+struct GraphMemory {
+    struct Block {
+        uint8_t* mem;
+        size_t bytes;
+        bool used;
+    };
+    std::mutex mu;
+    std::vector<Block> blocks;  // (never under `mu` while CUDA is called: user objects are released on CUDA's own threads)
+};
 
 struct bpq4k_context {
     int device = 0;
@@ -23,18 +39,29 @@ struct bpq4k_context {
     int prefill_arg() const { return prefill_mode | (prefill_variant << 4); }  // what the launcher takes
     int prefill_min_m = 25;  // four 8-row slabs of the streaming kernel cost as much as one tensor-core pass
     int rows_min_m = 0;  // 0: automatic; smallest M of the several-rows kernel (takes_rows_kernel)
-    // its workspaces, one per stream that uses it (overlapping calls on two streams must not share one): counters and
-    // the buffer of calls of up to kRowsFixedM rows; two are allocated with the handle (a program's stream and the one it
-    // captures graphs on), two more when needed
-    static constexpr uint32_t kRowsFixedM = 64;
-    static constexpr size_t kRowsCounterBytes = 1024;
-    struct RowsWorkspace {
+    // Its working memory.  The first streams that make such calls keep a block each (the stream's identity, which is never
+    // used again, tells them apart, not its handle); other streams' calls take theirs from the pool in stream order, which
+    // costs a call about a microsecond.  Calls that are captured have memory of their own, which follows the graph.
+    cudaMemPool_t rows_pool = nullptr;
+    size_t rows_keep = 0;  // what the pool keeps when a stream is waited for: twice the largest call so far
+    struct StreamBlock {
+        unsigned long long stream = 0;
         uint8_t* mem = nullptr;
-        cudaStream_t stream = nullptr;
-        bool assigned = false;
+        size_t bytes = 0;
     };
-    static constexpr uint32_t kRowsWorkspaces = 4;
-    RowsWorkspace rows_ws[kRowsWorkspaces];
+    static constexpr uint32_t kStreamBlocks = 2;
+    static constexpr size_t kRowsFirstBytes = 16u << 20;  // (24 rows of K = 28672 need 11 MB); mapped when the handle is made
+    StreamBlock stream_blocks[kStreamBlocks];
+    std::shared_ptr<GraphMemory> graph_memory;
+    struct CaptureEntry {
+        unsigned long long capture = 0;
+        cudaStream_t stream = nullptr;
+        uint8_t* mem = nullptr;
+        size_t bytes = 0;
+    };
+    static constexpr uint32_t kCaptureEntries = 8;
+    CaptureEntry captures[kCaptureEntries];  // the last captures' blocks
+    uint32_t next_capture = 0;
     uint64_t launches = 0;
     // staging for the *_host entry point
     float* stage_x = nullptr;
@@ -161,34 +188,82 @@ constexpr uint32_t kStreamMaxM = 16;  // rows of X one streaming launch can cove
 // two slabs of 8 read from shared memory: 304 against 199 us on 128256 x 4096).
 inline uint32_t stream_slab_rows(uint32_t K) { return (uint64_t)K * 16u * 4u <= 132u * 1024u ? 16u : 8u; }
 
-int alloc_rows_workspace(bpq4k_context::RowsWorkspace& w) {
-    const size_t bytes = bpq4k_context::kRowsCounterBytes + rows_buffer_bytes(bpq4k_context::kRowsFixedM, kRowsMaxK);
-    if (cudaMalloc(reinterpret_cast<void**>(&w.mem), bytes) == cudaSuccess) return BPQ4K_OK;  // (each call clears its counters itself)
-    cudaGetLastError();
-    w.mem = nullptr;
-    return BPQ4K_ERR_ALLOC;
+// Memory calls are allowed, for the scope's duration, while this thread captures a stream in whatever mode.
+struct AllocWhileCapturing {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+struct GraphHold {  // what a graph's user object refers to
+    std::shared_ptr<GraphMemory> memory;
+    uint8_t* mem;
+};
+void CUDART_CB release_graph_hold(void* p) {
+    GraphHold* hold = static_cast<GraphHold*>(p);
+    {
+        std::lock_guard<std::mutex> lock(hold->memory->mu);
+        for (auto& b : hold->memory->blocks)
+            if (b.mem == hold->mem) b.used = false;
+    }
+    delete hold;
 }
 
-// The several-rows kernel's workspace for calls on `st`; null: none left (or none can be allocated while `st` is being
-// captured), and the caller takes the other kernels.
-uint8_t* rows_workspace(bpq4k_context* h, cudaStream_t st) {
-    for (auto& w : h->rows_ws)
-        if (w.assigned && w.stream == st) return w.mem;
-    for (auto& w : h->rows_ws) {
-        if (w.assigned) continue;
-        if (!w.mem) {
-            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-                cudaGetLastError();
-                return nullptr;
-            }
-            if (alloc_rows_workspace(w) != BPQ4K_OK) return nullptr;
+// A block of at least `need` bytes for calls that stream `st` records into `graph`.  Calls recorded on one stream run one
+// after the other and share a block; each fork of a capture has its own.  Null: no memory.
+uint8_t* graph_block(bpq4k_context* h, cudaStream_t st, unsigned long long capture, cudaGraph_t graph, size_t need) {
+    size_t want = need;
+    for (const auto& c : h->captures)
+        if (c.mem && c.capture == capture && c.stream == st) {
+            if (c.bytes >= need) return c.mem;
+            if (want < 2 * c.bytes) want = 2 * c.bytes;  // (the smaller block stays with the graph, whose earlier calls use it)
         }
-        w.assigned = true;
-        w.stream = st;
-        return w.mem;
+    AllocWhileCapturing allow;
+    GraphMemory& gm = *h->graph_memory;
+    uint8_t* mem = nullptr;
+    size_t bytes = 0;
+    {
+        std::lock_guard<std::mutex> lock(gm.mu);
+        GraphMemory::Block* best = nullptr;
+        for (auto& b : gm.blocks)
+            if (!b.used && b.bytes >= need && (!best || b.bytes < best->bytes)) best = &b;
+        if (best) best->used = true, mem = best->mem, bytes = best->bytes;
     }
-    return nullptr;
+    if (!mem) {
+        if (cudaMalloc(reinterpret_cast<void**>(&mem), want) != cudaSuccess) {
+            cudaGetLastError();
+            return nullptr;
+        }
+        bytes = want;
+        bool listed = true;
+        try {
+            std::lock_guard<std::mutex> lock(gm.mu);
+            gm.blocks.push_back({mem, bytes, true});
+        } catch (const std::bad_alloc&) {
+            listed = false;
+        }
+        if (!listed) {
+            cudaFree(mem);
+            return nullptr;
+        }
+    }
+    GraphHold* hold = new (std::nothrow) GraphHold{h->graph_memory, mem};
+    cudaUserObject_t object = nullptr;
+    if (!hold || cudaUserObjectCreate(&object, hold, release_graph_hold, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        delete hold;
+        std::lock_guard<std::mutex> lock(gm.mu);
+        for (auto& b : gm.blocks)
+            if (b.mem == mem) b.used = false;
+        return nullptr;
+    }
+    if (cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(object, 1);  // gives the block back
+        return nullptr;
+    }
+    h->captures[h->next_capture++ % bpq4k_context::kCaptureEntries] = {capture, st, mem, bytes};
+    return mem;
 }
 
 // Which Q4_K / Q5_K calls take the several-rows kernel.  To 8 rows the streaming kernel reads the
@@ -219,39 +294,63 @@ bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a, int qtype) {
 }
 
 // One call of the several-rows kernel.  cudaErrorInvalidValue: it cannot serve the call (form, shape or memory), and the
-// caller takes the other kernels.  More than kRowsFixedM rows use the handle's scratch as the prefill kernel does.
-// `owner`: the stream in whose order the call runs, where that is not `st` itself.
-cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, cudaStream_t owner, int qtype, int* launches) {
+// caller takes the other kernels.
+cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, int qtype, int* launches) {
     if (!takes_rows_kernel(h, a, qtype)) return cudaErrorInvalidValue;
-    uint8_t* ws = rows_workspace(h, owner);
-    if (!ws) return cudaErrorInvalidValue;
-    void* buffer = ws + bpq4k_context::kRowsCounterBytes;
-    const size_t need = rows_buffer_bytes(a.M, a.K);
-    size_t have = rows_buffer_bytes(bpq4k_context::kRowsFixedM, kRowsMaxK);
-    if (a.M > bpq4k_context::kRowsFixedM) {
-        if (need > h->scratch_bytes) {
-            // nothing may be allocated while the stream is being captured; the prefill kernel may need less
-            cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-                ensure_bytes(h, &h->scratch, &h->scratch_bytes, need) != BPQ4K_OK) {
-                cudaGetLastError();
-                return cudaErrorInvalidValue;
-            }
-        }
-        buffer = h->scratch;
-        have = h->scratch_bytes;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long capture = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(st, &status, &capture, &graph, nullptr, nullptr) != cudaSuccess || status == cudaStreamCaptureStatusInvalidated) {
+        cudaGetLastError();
+        return cudaErrorInvalidValue;
     }
-    return launch_rows_tc(a, reinterpret_cast<uint32_t*>(ws), buffer, have, h->dev_status, h->sm_count, &h->tmaps, !h->tune.no_pdl,
-                          st, launches, qtype);
+    const size_t need = rows_buffer_bytes(a.M, a.K);
+    void* buffer = nullptr;
+    if (status == cudaStreamCaptureStatusActive) {
+        buffer = graph_block(h, st, capture, graph, need);
+        if (!buffer) return cudaErrorInvalidValue;
+        return launch_rows_tc(a, buffer, need, h->dev_status, h->sm_count, &h->tmaps, !h->tune.no_pdl, st, launches, qtype);
+    }
+    unsigned long long id = 0;
+    if (cudaStreamGetId(st, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaErrorInvalidValue;
+    }
+    bpq4k_context::StreamBlock* own = nullptr;
+    for (auto& b : h->stream_blocks)
+        if (b.mem && b.stream == id) own = &b;
+    for (auto& b : h->stream_blocks)
+        if (!own && !b.mem) own = &b;
+    if (own && own->bytes >= need)
+        return launch_rows_tc(a, own->mem, need, h->dev_status, h->sm_count, &h->tmaps, !h->tune.no_pdl, st, launches, qtype);
+    AllocWhileCapturing allow;  // (another stream may be captured meanwhile)
+    if (2 * need > h->rows_keep) {
+        uint64_t keep = h->rows_keep = 2 * need;
+        cudaMemPoolSetAttribute(h->rows_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    size_t bytes = need;
+    if (own) {
+        if (own->mem) cudaFreeAsync(own->mem, st);  // (it is this stream's)
+        *own = {};
+        if (bytes < bpq4k_context::kRowsFirstBytes) bytes = bpq4k_context::kRowsFirstBytes;
+    }
+    if (cudaMallocFromPoolAsync(&buffer, bytes, h->rows_pool, st) != cudaSuccess) {
+        cudaGetLastError();
+        return cudaErrorInvalidValue;
+    }
+    if (own) *own = {id, static_cast<uint8_t*>(buffer), bytes};
+    const cudaError_t e = launch_rows_tc(a, buffer, need, h->dev_status, h->sm_count, &h->tmaps, !h->tune.no_pdl, st, launches, qtype);
+    if (own) return e;
+    const cudaError_t f = cudaFreeAsync(buffer, st);
+    return e != cudaSuccess ? e : f;
 }
 
 // Kernel selection.  FP32: always the float kernel.  STREAM / AUTO: the streaming
 // kernel, X walked in slabs of 8 rows (each slab re-reads the weights, as the
 // reference's batched8 shader does per 8 rows).
-// `owner`: the stream in whose order the call runs, where that is not `st` itself.
-int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, cudaStream_t owner) {
+int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
     int launches = 0;
-    cudaError_t e = run_rows(h, a, st, owner, BPQ4K_TYPE_Q4_K, &launches);
+    cudaError_t e = run_rows(h, a, st, BPQ4K_TYPE_Q4_K, &launches);
     if (e != cudaErrorInvalidValue) {
         h->launches += (uint64_t)launches;
         if (e == cudaSuccess) return BPQ4K_OK;
@@ -346,14 +445,34 @@ int bpq4k_create(int device, bpq4k_handle_t* out) {
             e2 = cudaMalloc(&h->scratch, 4u << 20);
             if (e2 == cudaSuccess) h->scratch_bytes = 4u << 20;
         }
-        for (int i = 0; i < 2 && e2 == cudaSuccess; i++)
-            if (alloc_rows_workspace(h->rows_ws[i]) != BPQ4K_OK) e2 = cudaErrorMemoryAllocation;
+        if (e2 == cudaSuccess) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            e2 = cudaMemPoolCreate(&h->rows_pool, &props);
+            int no = 0;  // a stream takes another's block only when that is free already: it never waits for the other stream
+            if (e2 == cudaSuccess) e2 = cudaMemPoolSetAttribute(h->rows_pool, cudaMemPoolReuseAllowInternalDependencies, &no);
+            uint64_t keep = h->rows_keep = bpq4k_context::kRowsFirstBytes;
+            if (e2 == cudaSuccess) e2 = cudaMemPoolSetAttribute(h->rows_pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            void* first = nullptr;  // (mapping it takes half a millisecond; without room for it calls take the other kernels)
+            if (e2 == cudaSuccess && cudaMallocFromPoolAsync(&first, bpq4k_context::kRowsFirstBytes, h->rows_pool, nullptr) == cudaSuccess)
+                cudaFreeAsync(first, nullptr);
+            if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(nullptr);
+            cudaGetLastError();
+        }
+        if (e2 == cudaSuccess) {
+            try {
+                h->graph_memory = std::make_shared<GraphMemory>();
+            } catch (const std::bad_alloc&) {
+                e2 = cudaErrorMemoryAllocation;
+            }
+        }
         if (e2 != cudaSuccess) {
             cudaGetLastError();
             if (h->dev_status) cudaFree(h->dev_status);
             if (h->scratch) cudaFree(h->scratch);
-            for (auto& w : h->rows_ws)
-                if (w.mem) cudaFree(w.mem);
+            if (h->rows_pool) cudaMemPoolDestroy(h->rows_pool);
             delete h;
             return BPQ4K_ERR_ALLOC;
         }
@@ -371,8 +490,16 @@ int bpq4k_destroy(bpq4k_handle_t h) {
         if (h->scratch) cudaFree(h->scratch);
         if (h->dev_status) cudaFree(h->dev_status);
         if (h->tune.stamps) cudaFree(h->tune.stamps);
-        for (auto& w : h->rows_ws)
-            if (w.mem) cudaFree(w.mem);
+        cudaDeviceSynchronize();  // (freeing a pool's memory by address waits for nothing)
+        for (auto& b : h->stream_blocks)
+            if (b.mem) cudaFree(b.mem);
+        if (h->rows_pool) cudaMemPoolDestroy(h->rows_pool);
+        std::vector<GraphMemory::Block> blocks;
+        {
+            std::lock_guard<std::mutex> lock(h->graph_memory->mu);
+            blocks.swap(h->graph_memory->blocks);
+        }
+        for (const auto& b : blocks) cudaFree(b.mem);
         for (uint32_t i = 0; i < h->n_retired; i++) cudaFree(h->retired[i]);
         if (h->batch_exec) cudaGraphExecDestroy(h->batch_exec);
         if (h->batch_stream) cudaStreamDestroy(h->batch_stream);
@@ -622,7 +749,7 @@ int bpq4k_matmul_f32(bpq4k_handle_t h, const float* X, const void* W, const floa
     a.N = N;
     a.K = K;
     a.w_row_bytes = (uint64_t)rowStrideWords * 4u;
-    return run_matmul(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream));
+    return run_matmul(h, a, static_cast<cudaStream_t>(stream));
 }
 
 // ---- Q5_K / Q6_K siblings ----------------------------------------------------
@@ -736,7 +863,7 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
     int launches = 0;
     cudaError_t e = cudaErrorInvalidValue;
     if (qtype == BPQ4K_TYPE_Q5_K) {
-        e = run_rows(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream), qtype, &launches);
+        e = run_rows(h, a, static_cast<cudaStream_t>(stream), qtype, &launches);
         if (e != cudaErrorInvalidValue) {
             h->launches += (uint64_t)launches;
             if (e == cudaSuccess) return BPQ4K_OK;
@@ -885,7 +1012,7 @@ int bpq4k_matmul_moe_f32(bpq4k_handle_t h, const float* X, const void* W, const 
     a.x_rows = x_rows;
     a.n_slots = nSlots;
     a.w_total_rows = wRows;
-    return run_matmul(h, a, static_cast<cudaStream_t>(stream), static_cast<cudaStream_t>(stream));
+    return run_matmul(h, a, static_cast<cudaStream_t>(stream));
 }
 
 int bpq4k_kq_matmul_moe_f32(bpq4k_handle_t h, int qtype, const float* X, const void* W, const float* bias, float* Y,
@@ -1040,7 +1167,7 @@ int bpq4k_matmul_host_f32(bpq4k_handle_t h, const float* X_host, const void* W_d
     a.N = N;
     a.K = K;
     a.w_row_bytes = (uint64_t)rowStrideWords * 4u;
-    if (int s = run_matmul(h, a, st, st)) return s;
+    if (int s = run_matmul(h, a, st)) return s;
     e = cudaMemcpyAsync(Y_host, h->stage_y, yb, cudaMemcpyDeviceToHost, st);
     if (e != cudaSuccess) return cuda_fail(h, e, "result read-back");
     e = cudaStreamSynchronize(st);
@@ -1283,7 +1410,7 @@ int bpq4k_matmul_host_batch_f32(bpq4k_handle_t h, const bpq4k_host_matmul* items
             a.N = it.N;
             a.K = it.K;
             a.w_row_bytes = (uint64_t)it.rowStrideWords * 4u;
-            if (int s = run_matmul(h, a, s_, st)) return s;  // (recorded on the handle's own stream, replayed in the order of st)
+            if (int s = run_matmul(h, a, s_)) return s;
             xo += ((size_t)it.M * it.K * 4u + 255u) & ~(size_t)255u;
             yo += ((size_t)it.M * it.N * 4u + 255u) & ~(size_t)255u;
         }

@@ -149,12 +149,12 @@ size_t prefill_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int mode, int s
 cudaError_t launch_prefill_tc(const MatmulArgs& a, int mode, void* scratch, size_t scratch_bytes, int* status_dev,
                               int sm_count, cudaStream_t stream, int* launches, int qtype = 12);  // 12 Q4_K, 13 Q5_K, 0x10E padded Q6_K
 
-// Matmul of several activation rows, K up to 32768 (q4k_rows_tc.cu), two or three launches.  `counters`: 160 words,
-// `buffer`: rows_buffer_bytes() bytes; what they hold before a call does not matter, and both serve one call at a time.
+// Matmul of several activation rows, K up to 32768 (q4k_rows_tc.cu), two or three launches.  `buffer`: rows_buffer_bytes()
+// bytes, 256-byte aligned; what it holds before a call does not matter, and it serves one call at a time.
 // cudaErrorInvalidValue: not a shape or form of this kernel.
 constexpr uint32_t kRowsMaxM = 16384, kRowsMaxK = 32768;
 size_t rows_buffer_bytes(uint32_t M, uint32_t K);
-cudaError_t launch_rows_tc(const MatmulArgs& a, uint32_t* counters, void* buffer, size_t buffer_bytes, int* status_dev,
+cudaError_t launch_rows_tc(const MatmulArgs& a, void* buffer, size_t buffer_bytes, int* status_dev,
                            int sm_count, TmapCache* tmaps, bool pdl, cudaStream_t stream, int* launches, int qtype = 12);
 
 // Cross-GPU barrier on flag words in peer memory (one process per GPU): store `epoch` into slot

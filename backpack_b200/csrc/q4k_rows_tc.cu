@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     const uint32_t c_last = unit_owner((dtile + 1u) * a.nsb - 1u, a.u_base, a.u_extra);
                     __threadfence();
                     asm volatile("bar.sync 1, %0;" ::"n"(kWorkers * 32) : "memory");
-                    if (threadIdx.x == 4u * 32u) *last_flag = atomicAdd(a.counters + c_first, 1u);
+                    if (threadIdx.x == 4u * 32u) *last_flag = atomicInc(a.counters + c_first, c_last - c_first);
                     asm volatile("bar.sync 1, %0;" ::"n"(kWorkers * 32) : "memory");
                     write = *last_flag == c_last - c_first;  // this CTA is the tile's last: add the segments in order of k
                     if (write) {
@@ -933,8 +933,10 @@ cudaError_t launch_rows_t(uint32_t T, const RowsArgs& ra, uint32_t grid, bool pd
 
 }  // namespace
 
-// Buffer of a call: the activation scales (2^-e), the image, two cut tiles per CTA.
-static size_t rows_head_bytes(uint32_t M) { return ((size_t)M * 4u + 127u + 256u) & ~(size_t)255u; }
+// Buffer of a call: the counters, the activation scales (2^-e), the image, two cut tiles per CTA.
+constexpr size_t kCounterBytes = 1024;
+static_assert(kCounterBytes >= kMaxCtas * 4u, "counters");
+static size_t rows_head_bytes(uint32_t M) { return kCounterBytes + (((size_t)M * 4u + 127u + 256u) & ~(size_t)255u); }
 static size_t rows_image_bytes(uint32_t M, uint32_t K) {
     const uint32_t T = rows_tile(M), tiles = (M + T - 1u) / T;
     return (size_t)tiles * T * (K / kQK) * 1088u;
@@ -945,19 +947,19 @@ static size_t rows_part_bytes(uint32_t M) {
 }
 size_t rows_buffer_bytes(uint32_t M, uint32_t K) { return rows_head_bytes(M) + rows_image_bytes(M, K) + rows_part_bytes(M); }
 
-cudaError_t launch_rows_tc(const MatmulArgs& m, uint32_t* counters, void* buffer, size_t buffer_bytes, int* status_dev, int sm_count,
+cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_bytes, int* status_dev, int sm_count,
                            TmapCache* tmaps, bool pdl, cudaStream_t stream, int* launches, int qtype) {
     if (m.M == 0 || m.N == 0) return cudaSuccess;
     if ((qtype != 12 && qtype != 13) || m.n_slots || m.n_peers || m.prologue || m.residual || m.M > kRowsMaxM || m.K > kRowsMaxK ||
-        !counters || !buffer || buffer_bytes < rows_buffer_bytes(m.M, m.K))
+        !buffer || buffer_bytes < rows_buffer_bytes(m.M, m.K))
         return cudaErrorInvalidValue;
     const bool q5 = qtype == 13;
     const uint32_t nsb = m.K / kQK, block_words = q5 ? 44u : 36u, T = rows_tile(m.M);
     const uint32_t tok_tiles = (m.M + T - 1u) / T;
     uint8_t* buf = static_cast<uint8_t*>(buffer);
     RowsArgs ra{};
-    ra.counters = counters;
-    ra.inv = reinterpret_cast<const float*>(buf);
+    ra.counters = reinterpret_cast<uint32_t*>(buf);
+    ra.inv = reinterpret_cast<const float*>(buf + kCounterBytes);
     ra.image = buf + rows_head_bytes(m.M);
     ra.part = reinterpret_cast<float*>(buf + rows_head_bytes(m.M) + rows_image_bytes(m.M, m.K));
     ra.tok_tiles = tok_tiles;
@@ -1014,7 +1016,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, uint32_t* counters, void* buffer
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv), counters);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv), ra.counters);
     if (launches) ++*launches;
     if (e != cudaSuccess) return e;
     e = q5 ? launch_rows_t<1>(T, ra, grid, pdl, stream) : launch_rows_t<0>(T, ra, grid, pdl, stream);

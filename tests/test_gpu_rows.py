@@ -117,39 +117,46 @@ def test_rows_kernel_not_finite_stays_in_its_row(ctx):
 
 
 def test_rows_kernel_threshold_streams_and_capture(ctx):
-    """Below the option's row count the streaming kernel runs; calls on several streams at once keep their own workspace;
-    a captured call replays."""
+    """Below the option's row count the streaming kernel runs; calls on several streams at once keep memory of their own, and
+    each of them runs this kernel (three launches; the streaming kernel takes one); a captured call replays."""
     import torch
 
     M, N, K = 12, 1000, 2048
     raw, w64 = make(q4k.Q4_K, N, K, 11)
     w = upload(ctx, q4k.Q4_K, raw, N, K)
-    xs = [synth.make_activations(M, K, 20 + i) for i in range(6)]
+    xs = [synth.make_activations(M, K, 20 + i) for i in range(10)]
     default = ctx.get_option(q4k.OPT_ROWS_MIN_M)
     try:
         ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)
+        ctx.launch_count(reset=True)
         close(ctx.matmul(torch.from_numpy(xs[0]).cuda(), w).cpu().numpy(), xs[0], w64)
+        assert ctx.launch_count() == 1
     finally:
         ctx.set_option(q4k.OPT_ROWS_MIN_M, default)
     xd = [torch.from_numpy(x).cuda() for x in xs]
+    want = [ctx.matmul(x, w) for x in xd]
     ys = [torch.empty(M, N, device="cuda") for _ in xs]
     streams = [torch.cuda.Stream() for _ in xs]
     torch.cuda.synchronize()
+    ctx.launch_count(reset=True)
     for _ in range(20):
         for x, y, s in zip(xd, ys, streams):
             with torch.cuda.stream(s):
                 ctx.matmul(x, w, out=y)
     torch.cuda.synchronize()
-    for x, y in zip(xs, ys):
+    assert ctx.launch_count() == 3 * 20 * len(xs)
+    for x, y, v in zip(xs, ys, want):
         close(y.cpu().numpy(), x, w64)
+        assert torch.equal(y, v)              # whichever stream a call runs on
     import backpack_b200 as bp
 
     c = bp.Q4KContext(0)
     try:
         y = torch.empty(M, N, device="cuda")
         g = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(g):             # the handle's first call: everything it needs was allocated with it
+        with torch.cuda.graph(g):             # the handle's first call
             c.matmul(xd[0], w, out=y)
+        assert c.launch_count() == 3
         for x in (1, 2):
             xd[0].copy_(xd[x])
             g.replay()
@@ -157,6 +164,147 @@ def test_rows_kernel_threshold_streams_and_capture(ctx):
             close(y.cpu().numpy(), xs[x], w64)
         assert c.device_status() == 0
         del g
+    finally:
+        c.close()
+
+
+@pytest.fixture(scope="module")
+def wide(ctx):
+    """Calls long enough to overlap: a weight matrix and two activations with their results."""
+    import torch
+
+    M, N, K = 13, 28672, 4096
+    w = upload(ctx, q4k.Q4_K, synth.make_q4k_weights(N, K, 61), N, K)
+    xs = [torch.from_numpy(synth.make_activations(M, K, 62 + i)).cuda() for i in range(2)]
+    ws = ctx.dequant(w).double()
+    want = [x.double() @ ws.T for x in xs]
+    return w, xs, want
+
+
+def same(y, v):
+    return float((y.double() - v).norm() / v.norm()) <= 4e-6
+
+
+@pytest.mark.parametrize("M", [13, 90])
+def test_rows_kernel_graphs_of_one_capture_stream_replay_side_by_side(ctx, M):
+    """Two graphs captured on one stream (torch's capture stream) and replayed on two, beside eager calls on a third."""
+    import torch
+
+    N, K = 28672, 4096
+    w = upload(ctx, q4k.Q4_K, synth.make_q4k_weights(N, K, 61), N, K)
+    xs = [torch.from_numpy(synth.make_activations(M, K, 62 + i)).cuda() for i in range(3)]
+    want = [ctx.matmul(x, w) for x in xs]
+    ys = [torch.zeros(M, N, device="cuda") for _ in xs]
+    graphs = []
+    capture = torch.cuda.Stream()
+    for x, y in zip(xs[:2], ys[:2]):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=capture):
+            for _ in range(4):
+                ctx.matmul(x, w, out=y)
+        graphs.append(g)
+    streams = [torch.cuda.Stream() for _ in xs]
+    torch.cuda.synchronize()
+    for _ in range(10):
+        for g, s in zip(graphs, streams):
+            with torch.cuda.stream(s):
+                g.replay()
+        for s in (streams[2], capture):
+            with torch.cuda.stream(s):
+                ctx.matmul(xs[2], w, out=ys[2])
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0
+    for y, v in zip(ys, want):
+        assert torch.equal(y, v)
+    del graphs
+
+
+def test_rows_kernel_batch_list_recorded_on_one_stream_and_called_on_another(ctx, wide):
+    """A list of host-buffer matmuls is recorded when it is called again, then replayed whatever the stream, beside work of
+    the stream it was recorded on."""
+    import torch
+
+    w, xs, want = wide
+    M, K = xs[0].shape
+    x_host = torch.empty(M, K, pin_memory=True)
+    x_host.copy_(xs[0])
+    y_host = torch.empty(M, w.N, pin_memory=True)
+    batch = ctx.make_host_batch([(x_host.numpy(), w, y_host.numpy(), None)])
+    streams = [torch.cuda.Stream() for _ in range(6)]
+    ys = [torch.empty(M, w.N, device="cuda") for _ in streams]
+    torch.cuda.synchronize()
+    records = ctx.get_option(q4k.OPT_BATCH_RECORDS)
+    for i in range(24):                       # (recorded on one of the first streams)
+        for s, y in zip(streams, ys):
+            with torch.cuda.stream(s):
+                for _ in range(3):
+                    ctx.matmul(xs[1], w, out=y)
+        y_host.zero_()
+        with torch.cuda.stream(streams[min(i, 23 - i) % 6]):
+            ctx.matmul_host_batch(batch)
+        assert same(y_host.cuda(), want[0]), i
+    assert ctx.get_option(q4k.OPT_BATCH_RECORDS) == records + 1
+    torch.cuda.synchronize()
+    assert ctx.device_status() == 0
+    for y in ys:
+        assert same(y, want[1])
+
+
+def test_rows_kernel_eager_call_beside_a_capture(ctx, wide):
+    """An eager call while another stream is captured (in the mode that forbids allocations) neither fails nor spoils it."""
+    import torch
+
+    w, xs, want = wide
+    ys = [torch.empty(xs[0].shape[0], w.N, device="cuda") for _ in xs]
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    import backpack_b200 as bp
+
+    c = bp.Q4KContext(0)                      # nothing allocated yet
+    try:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            c.matmul(xs[0], w, out=ys[0])
+            with torch.cuda.stream(other):
+                c.matmul(xs[1], w, out=ys[1])
+        g.replay()
+        torch.cuda.synchronize()
+        assert same(ys[0], want[0]) and same(ys[1], want[1])
+        del g
+    finally:
+        c.close()
+
+
+def test_rows_kernel_memory_of_handles_and_graphs(wide):
+    """A handle costs a few MB until a call needs more; memory of a captured call is used again once the graph is gone."""
+    import torch
+
+    import backpack_b200 as bp
+
+    w, xs, want = wide
+    torch.cuda.synchronize()
+    free0 = torch.cuda.mem_get_info()[0]
+    c = bp.Q4KContext(0)
+    try:
+        assert free0 - torch.cuda.mem_get_info()[0] <= 40 << 20   # (16 MB of working memory, 4 MB of scratch, the pool's granularity)
+        y = torch.empty(xs[0].shape[0], w.N, device="cuda")
+        free1 = None
+        for i in range(12):
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                c.matmul(xs[i % 2], w, out=y)
+            g.replay()
+            torch.cuda.synchronize()
+            assert same(y, want[i % 2])
+            g.reset()
+            del g
+            torch.cuda.synchronize()
+            import time
+
+            time.sleep(0.05)                  # (released on a thread of the driver's)
+            if i == 3:
+                free1 = torch.cuda.mem_get_info()[0]
+        assert torch.cuda.mem_get_info()[0] >= free1 - (4 << 20)
     finally:
         c.close()
 
