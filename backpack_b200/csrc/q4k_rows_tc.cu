@@ -37,6 +37,7 @@
 #include <cuda_fp16.h>
 
 #include <cstring>
+#include <type_traits>
 
 #include "kernels.h"
 #include "q4k_common.cuh"
@@ -51,11 +52,13 @@ constexpr uint32_t kMaxCtas = 160;                    // counters (one per CTA)
 constexpr uint32_t kWorkers = 16;                     // warps that dequantise and drain
 constexpr uint32_t kThreads = (4 + kWorkers) * 32;
 constexpr uint32_t kTileRows = 256;                   // weight rows of a unit: two row tiles of 128 lanes
+constexpr float kLowScale = 2048.f, kLowScaleInv = 1.f / 2048.f;  // of stacked low halves
 constexpr uint32_t kASlotCols = 40;                   // tensor-memory columns of one dequantised group: 32 codes + 8 (constant term)
 
 // T: activation rows of the tile.
 //   up to 32   the high and the low halves of the activations are stacked into one mma of 2T columns, each half with its
-//              own accumulator; above that they accumulate into the same T columns
+//              own accumulator; above that they accumulate into the same T columns.  Stacked low halves carry a factor 2^11 of
+//              their own (rows_pack_kernel)
 //   up to 48   two accumulators per row tile: the next super-block accumulates while the last is drained
 //   above      (WIDE) one accumulator per row tile (tensor memory holds two tiles' accumulators and the operand ring) and an issuing warp for each, the second two groups behind the
 //              first, so that one accumulates while the other is drained.  The T partial sums of a weight row fill a
@@ -91,6 +94,9 @@ struct RowsArgs {
     CUtensorMap tmap_w;       // [N rows][K/256 blocks] as 32-bit words, box 128 rows x 1 block
     const uint8_t* image;     // activation image (rows_pack_kernel)
     const float* inv;         // 2^-e per activation row
+    const float* sb_scale;    // STACK: [super-block][T], read only if a word of `spread` is not zero
+    const uint32_t* spread;
+    uint32_t n_spread;
     const float* bias;
     float* Y;
     uint32_t M, N, nsb, u_base, u_extra;
@@ -193,6 +199,9 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* v) {
     asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]),
                  "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
+}
+__device__ __forceinline__ void ldg128(const float* p, float* v) {
+    asm volatile("ld.global.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]) : "l"(p) : "memory");
 }
 template <int C>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t* v) {
@@ -626,13 +635,21 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
         float y[TH];
 #pragma unroll
         for (int j = 0; j < TH; j++) y[j] = 0.f;
+        // The low halves' own sum, or one fma more a super-block: which is faster is the compiler's schedule (57344 x 8192, us,
+        // two sums | one: 8 rows 86.4 | 87.7, 16 rows 95.7 | 89.9, 24 rows 95.1 | 97.8).
+        constexpr bool TWO_SUMS = P::STACK && T <= 24 && T != 16;
+        [[maybe_unused]] float yl[TWO_SUMS ? TH : 1];
+        if constexpr (TWO_SUMS)
+#pragma unroll
+            for (int j = 0; j < TH; j++) yl[j] = 0.f;
         float s_prev = 0.f;
         uint32_t dtile = u0 / a.nsb, db = u0 - dtile * a.nsb;  // of the super-block that is drained next
         bool seg_head = db == 0;                             // its segment starts at its tile's first block
         uint32_t rs = rt, rit = 0;                          // raw ring position (stages alternate between the row tiles)
         uint32_t sa = set, ita = 0;                         // operand ring position (groups alternate between the sets)
 
-        auto drain = [&](uint32_t kd) {
+        auto drain = [&](uint32_t kd, auto spread) {
+            constexpr bool SPREAD = decltype(spread)::value;
             const uint32_t buf = kd % P::NBUF;
             wait_bar(acc_full(rt, buf), (kd / P::NBUF) & 1u, abort_flag, a.status);
             __syncwarp();
@@ -649,15 +666,35 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(acc_empty(rt, buf));
+            if constexpr (SPREAD) {  // (stacked, one activation tile)
 #pragma unroll
-            for (int j = 0; j < TH; j++) {
-                float v = __uint_as_float(hi[j]);
-                if constexpr (P::STACK) v += __uint_as_float(lo[j]);
-                y[j] = fmaf(s_prev, v, y[j]);
+                for (int c = 0; c < TH; c += 4) {
+                    float f[4];
+                    ldg128(a.sb_scale + db * T + set * TH + c, f);
+#pragma unroll
+                    for (int j = 0; j < 4; j++)
+                        y[c + j] = fmaf(s_prev, fmaf(__uint_as_float(lo[c + j]), kLowScaleInv, __uint_as_float(hi[c + j])) * f[j], y[c + j]);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < TH; j++) {
+                    if constexpr (TWO_SUMS) {
+                        y[j] = fmaf(s_prev, __uint_as_float(hi[j]), y[j]);
+                        yl[j] = fmaf(s_prev, __uint_as_float(lo[j]), yl[j]);
+                    } else if constexpr (P::STACK) {
+                        y[j] = fmaf(s_prev, fmaf(__uint_as_float(lo[j]), kLowScaleInv, __uint_as_float(hi[j])), y[j]);
+                    } else {
+                        y[j] = fmaf(s_prev, __uint_as_float(hi[j]), y[j]);
+                    }
+                }
             }
             const bool tile_end = db + 1u == a.nsb;
             if (tile_end || kd + 1u == nu) {
                 // ---- end of a segment: a whole tile goes to Y, a cut one to the workspace ----
+                if constexpr (TWO_SUMS) {
+#pragma unroll
+                    for (int j = 0; j < TH; j++) y[j] = fmaf(yl[j], kLowScaleInv, y[j]), yl[j] = 0.f;
+                }
                 asm volatile("griddepcontrol.wait;" ::: "memory");
                 const uint32_t rtile = dtile / a.tok_tiles, tok0 = (dtile - rtile * a.tok_tiles) * T;
                 const uint32_t n = rtile * kTileRows + rt * 128u + row;
@@ -712,7 +749,8 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
             else db++;
         };
 
-        for (uint32_t k = 0; k <= nu; k++) {
+        auto turns = [&](uint32_t k0, uint32_t k1, auto spread) {
+            for (uint32_t k = k0; k < k1; k++) {
             const bool more = k < nu;
             BlockScales h;
             if (more) {
@@ -755,8 +793,20 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     if (sa >= P::NA) sa -= P::NA, ita++;
                 }
             }
-            if (k > 0) drain(k - 1u);
+            if (k > 0) drain(k - 1u, spread);
             s_prev = h.s;
+            }
+        };
+        if constexpr (P::STACK) {
+            // the first drain needs to know whether some super-block of some row has a scale of its own
+            turns(0, 1, std::false_type{});
+            asm volatile("griddepcontrol.wait;" ::: "memory");
+            uint32_t any = 0;
+            for (uint32_t i = lane; i < a.n_spread; i += 32u) any |= __ldcg(a.spread + i);
+            if (__any_sync(0xFFFFFFFFu, any != 0u)) turns(1, nu + 1u, std::true_type{});
+            else turns(1, nu + 1u, std::false_type{});
+        } else {
+            turns(0, nu + 1u, std::false_type{});
         }
         fence_before();
     }
@@ -768,7 +818,12 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 }
 
 // Activations -> the image the matmul copies tile by tile.  Row t is scaled by a power of two that brings its largest
-// magnitude into [2^14, 2^15) and split into halves (values down to 2^-30 of the largest keep 2^-10 of themselves).  Per activation tile and super-block four groups of T*256 bytes: rows
+// magnitude into [2^14, 2^15) and split into halves.  Stacked (T <= 32): the low halves are scaled by 2^11 more, so that they
+// have a half's whole range below them, and a super-block whose largest lies 2^4 or more below the row's is scaled by a power
+// of its own (`spread` says that there is one; the drain then applies the powers, 3 to 5 % slower): a value keeps 22 bits down to
+// 2^-24 of its super-block's largest, where the streaming kernel, which serves fewer rows, keeps 21 of the largest of 32.  Not
+// stacked: 22 bits down to 2^-17 of the row's largest, 2^-39 of that below (the prefill kernel, which served these rows before,
+// 2^-25 whatever the row).  Per activation tile and super-block four groups of T*256 bytes: rows
 // 0..T-1 the high halves, T..2T-1 the low ones, 128 B each in the 128-byte swizzle, a 16-byte chunk i holding the
 // activations of code word i in the order the dequantiser produces its weights (4i, 4i+2, 4i+1, 4i+3 of the even
 // sub-block, then of the odd one); then the same rows with 32 B each: the mean of each of the eight sub-blocks, twice
@@ -779,6 +834,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 // held before it (a clear by another stream's memset would not be ordered against the kernel).
 __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict__ X, uint32_t M, uint32_t K, uint32_t T,
                                                         uint8_t* __restrict__ image, float* __restrict__ inv,
+                                                        float* __restrict__ sb_scale, uint32_t* __restrict__ spread,
                                                         uint32_t* __restrict__ counters) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -788,7 +844,8 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
     const bool live = row < M;
     if (row == 0 && blockIdx.x == 0 && threadIdx.x < kMaxCtas) counters[threadIdx.x] = 0;
     const float4* x4 = reinterpret_cast<const float4*>(X + (uint64_t)row * K);
-    float scale = 0.f;
+    const bool stack = T <= 32u;
+    uint32_t e = 0;  // biased exponent of the row's scale
     if (live) {
         // magnitudes compare as integers; a NaN counts as larger than infinity and reaches every output of the row
         uint32_t mx = 0;
@@ -803,15 +860,15 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < 8; i++) mx = max(mx, red[i]);
-        uint32_t e = 268u - (mx >> 23);  // biased exponent of 2^14 / 2^exponent(mx)
-        if (e > 253u) e = 253u;
-        scale = __uint_as_float(e << 23);
+        e = min(268u - (mx >> 23), 253u);  // of 2^14 / 2^exponent(mx)
         if (blockIdx.x == 0 && threadIdx.x == 0) inv[row] = __uint_as_float((254u - e) << 23);
     }
-    auto split = [](float p, float q, uint32_t& h, uint32_t& l) {
+    int spread_any = 0;
+    const float low = stack ? kLowScale : 1.f;
+    auto split = [low](float p, float q, uint32_t& h, uint32_t& l) {
         h = half2_bits(p, q);
         const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
-        l = half2_bits(p - f.x, q - f.y);
+        l = half2_bits((p - f.x) * low, (q - f.y) * low);
     };
     const uint32_t g = lane >> 3, i = lane & 7u;
     for (uint32_t sb = blockIdx.x * 8u + warp; sb < nsb; sb += gridDim.x * 8u) {
@@ -819,6 +876,19 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
         if (live) {
             e4 = __ldg(x4 + sb * 64u + g * 16u + i);
             o4 = __ldg(x4 + sb * 64u + g * 16u + 8u + i);
+        }
+        uint32_t es = e;  // biased exponent of this super-block's scale
+        if (stack) {
+            auto mag = [](const float4& v) {
+                return max(max(__float_as_uint(v.x) & 0x7FFFFFFFu, __float_as_uint(v.y) & 0x7FFFFFFFu),
+                           max(__float_as_uint(v.z) & 0x7FFFFFFFu, __float_as_uint(v.w) & 0x7FFFFFFFu));
+            };
+            const uint32_t mx = __reduce_max_sync(0xFFFFFFFFu, max(mag(e4), mag(o4))), own = min(268u - (mx >> 23), 253u);
+            // (at most 2^100 beside the row's: the inverse stays an ordinary float)
+            if (mx && own >= e + 4u) es = min(own, e + 100u), spread_any = 1;
+        }
+        if (live) {
+            const float scale = __uint_as_float(es << 23);
             e4.x *= scale, e4.y *= scale, e4.z *= scale, e4.w *= scale;
             o4.x *= scale, o4.y *= scale, o4.z *= scale, o4.w *= scale;
         }
@@ -828,6 +898,7 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
         split(o4.x, o4.z, hi.z, lo.z);
         split(o4.y, o4.w, hi.w, lo.w);
         uint8_t* blk = image + ((uint64_t)tt * nsb + sb) * T * 1088u;
+        if (stack && lane == 0) sb_scale[((uint64_t)tt * nsb + sb) * T + t] = live ? __uint_as_float((127u + e - es) << 23) : 0.f;
         auto put = [&](uint32_t r, const uint4& v) { *reinterpret_cast<uint4*>(blk + g * T * 256u + r * 128u + ((i ^ (r & 7u)) << 4)) = v; };
         put(t, hi);
         put(T + t, lo);
@@ -841,6 +912,10 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
         split(0.03125f * se, 0.03125f * so, sh, sl);
         if (i < 4)  // two chunks of the high row, two of the low one
             *reinterpret_cast<uint32_t*>(blk + T * 1024u + (i < 2 ? t : T + t) * 32u + (i & 1u) * 16u + g * 4u) = i < 2 ? sh : sl;
+    }
+    if (stack) {
+        spread_any = __syncthreads_or(spread_any);
+        if (threadIdx.x == 0) spread[row * gridDim.x + blockIdx.x] = spread_any;
     }
 }
 
@@ -933,13 +1008,21 @@ cudaError_t launch_rows_t(uint32_t T, const RowsArgs& ra, uint32_t grid, bool pd
 
 }  // namespace
 
-// Buffer of a call: the counters, the activation scales (2^-e), the image, two cut tiles per CTA.
+// Blocks of rows_pack_kernel that share a row: one from four blocks per SM on, else as many as the row has warps' work for.
+static uint32_t pack_blocks(uint32_t rows, uint32_t nsb, uint32_t ctas) {
+    const uint32_t want = 4u * ctas / rows, most = (nsb + 7u) / 8u;
+    return want < 1u ? 1u : want < most ? want : most;
+}
+constexpr uint32_t kSpreadWords = 32u * (kRowsMaxK / kQK / 8u);
+
+// Buffer of a call: the counters, the activation scales (2^-e), the image, (to 32 rows) the words of `spread` and the
+// super-blocks' scales, two cut tiles per CTA.
 constexpr size_t kCounterBytes = 1024;
 static_assert(kCounterBytes >= kMaxCtas * 4u, "counters");
 static size_t rows_head_bytes(uint32_t M) { return kCounterBytes + (((size_t)M * 4u + 127u + 256u) & ~(size_t)255u); }
 static size_t rows_image_bytes(uint32_t M, uint32_t K) {
     const uint32_t T = rows_tile(M), tiles = (M + T - 1u) / T;
-    return (size_t)tiles * T * (K / kQK) * 1088u;
+    return (size_t)tiles * T * (K / kQK) * 1088u + (((T <= 32u ? kSpreadWords * 4u + (size_t)T * (K / kQK) * 4u : 0u) + 255u) & ~(size_t)255u);
 }
 static size_t rows_part_bytes(uint32_t M) {
     const uint32_t T = rows_tile(M);
@@ -956,11 +1039,15 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
     const bool q5 = qtype == 13;
     const uint32_t nsb = m.K / kQK, block_words = q5 ? 44u : 36u, T = rows_tile(m.M);
     const uint32_t tok_tiles = (m.M + T - 1u) / T;
+    const uint32_t ctas = (uint32_t)sm_count < kMaxCtas ? (uint32_t)sm_count : kMaxCtas;
     uint8_t* buf = static_cast<uint8_t*>(buffer);
     RowsArgs ra{};
     ra.counters = reinterpret_cast<uint32_t*>(buf);
     ra.inv = reinterpret_cast<const float*>(buf + kCounterBytes);
     ra.image = buf + rows_head_bytes(m.M);
+    ra.spread = reinterpret_cast<const uint32_t*>(ra.image + (size_t)tok_tiles * T * nsb * 1088u);
+    ra.sb_scale = reinterpret_cast<const float*>(ra.spread + kSpreadWords);
+    ra.n_spread = T <= 32u ? pack_blocks(tok_tiles * T, nsb, ctas) * T : 0u;
     ra.part = reinterpret_cast<float*>(buf + rows_head_bytes(m.M) + rows_image_bytes(m.M, m.K));
     ra.tok_tiles = tok_tiles;
     ra.slot_rows = m.M < T ? m.M : T;
@@ -973,7 +1060,6 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
     const uint64_t units64 = (uint64_t)((m.N + kTileRows - 1u) / kTileRows) * tok_tiles * nsb;
     if (units64 > 0x3FFFFFFFull) return cudaErrorInvalidValue;  // (group numbers stay below 2^32)
     const uint32_t units = (uint32_t)units64;
-    const uint32_t ctas = (uint32_t)sm_count < kMaxCtas ? (uint32_t)sm_count : kMaxCtas;
     const uint32_t grid = units < ctas ? units : ctas;
     ra.u_base = units / grid;
     ra.u_extra = units % grid;
@@ -1006,9 +1092,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
         }
     }
     cudaLaunchConfig_t cfg{};
-    // one block per row from four blocks per SM on, else as many as the row has warps' work for
-    const uint32_t rows = tok_tiles * T, want = 4u * ctas / rows, most = (nsb + 7u) / 8u;
-    cfg.gridDim = dim3(want < 1u ? 1u : want < most ? want : most, rows);
+    cfg.gridDim = dim3(pack_blocks(tok_tiles * T, nsb, ctas), tok_tiles * T);
     cfg.blockDim = dim3(256);
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -1016,7 +1100,8 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv), ra.counters);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv),
+                                       const_cast<float*>(ra.sb_scale), const_cast<uint32_t*>(ra.spread), ra.counters);
     if (launches) ++*launches;
     if (e != cudaSuccess) return e;
     e = q5 ? launch_rows_t<1>(T, ra, grid, pdl, stream) : launch_rows_t<0>(T, ra, grid, pdl, stream);

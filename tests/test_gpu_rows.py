@@ -101,6 +101,39 @@ def test_rows_kernel_range_of_activations_and_scales(ctx, M):
         assert np.all(np.abs(y[t] - want) <= bound), (t, np.max(np.abs(y[t] - want) / bound))
 
 
+@pytest.mark.parametrize("qtype", [q4k.Q4_K, q4k.Q5_K], ids=["q4_k", "q5_k"])
+@pytest.mark.parametrize("M", [3, 8, 16, 24, 32])
+@pytest.mark.parametrize("where,power", [("block", 20), ("block", 42), ("block", 80), ("sub", 17), ("sub", 24), ("sub", 28)])
+def test_rows_kernel_small_values_beside_large_ones(ctx, qtype, M, where, power):
+    """Activations 2^power below others of their row, whose weights are zero: in another super-block they keep all 22 bits
+    (a super-block whose largest lies 2^4 below the row's has a scale of its own), in the same one down to 2^-24 of its
+    largest: an error of 2^-36 of the scaled value, whose largest is at least 2^11, so 2^-47 * 2^28 = 2^-19 of a value at
+    2^-28.  `close` allows 4e-6 = 2^-18."""
+    import torch
+
+    N, K = 300, 1024
+    raw, _ = make(qtype, N, K, 51)
+    blocks = raw.reshape(N, K // 256, -1).copy()
+    x = synth.make_activations(M, K, 52)
+    small = x.copy()
+    if where == "block":
+        blocks[:, 1, :4] = 0                  # d and dmin
+        x[:, 256:512] *= np.float32(2.0**power)
+        small[:, 256:512] = 0.0
+    else:
+        blocks[:, :, 4 + 1] &= 0xC0           # scale and minimum of every second sub-block
+        blocks[:, :, 8 + 1] &= 0xC0
+        one = (np.arange(K) // 32) % 8 == 1
+        x[:, one] *= np.float32(2.0**power)
+        small[:, one] = 0.0
+    raw = blocks.reshape(-1)
+    w64 = (orc.dequant(raw, N, K) if qtype == q4k.Q4_K else orc.kq_dequant(orc.Q5_K, raw, N, K)).reshape(N, K).astype(np.float64)
+    y = ctx.matmul(torch.from_numpy(x).cuda(), upload(ctx, qtype, raw, N, K)).cpu().numpy()
+    assert ctx.device_status() == 0
+    assert (x.astype(np.float64) @ w64.T == small.astype(np.float64) @ w64.T).all()
+    close(y, small, w64)
+
+
 def test_rows_kernel_not_finite_stays_in_its_row(ctx):
     import torch
 
