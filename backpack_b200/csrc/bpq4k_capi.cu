@@ -62,6 +62,7 @@ struct bpq4k_context {
     static constexpr uint32_t kCaptureEntries = 8;
     CaptureEntry captures[kCaptureEntries];  // the last captures' blocks
     uint32_t next_capture = 0;
+    int last_kernel = BPQ4K_KERNEL_NONE;  // BPQ4K_OPT_LAST_MATMUL_KERNEL
     uint64_t launches = 0;
     // staging for the *_host entry point
     float* stage_x = nullptr;
@@ -276,9 +277,10 @@ uint8_t* graph_block(bpq4k_context* h, cudaStream_t st, unsigned long long captu
 bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a, int qtype) {
     if (h->gemv_variant != BPQ4K_GEMV_AUTO || a.n_slots || a.n_peers || !aligned16(a.X)) return false;
     const uint32_t min_m = h->rows_min_m ? (uint32_t)h->rows_min_m : a.K >= 8192u ? 5u : 9u;
-    if (a.M < min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u)) return false;
+    if (a.M < min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u && !h->rows_min_m)) return false;
     if (a.M < (uint32_t)h->prefill_min_m) return a.M <= 24u;
     if (h->prefill_mode != BPQ4K_PREFILL_F16X3) return false;
+    if (h->rows_min_m) return true;  // the caller's own threshold
     // Against the prefill kernel (us, prefill | here).  To 96 rows here: 80 rows, 6144 x 4096 33 | 26, 128256 x 4096 350 | 195.
     // To 128 rows where a CTA has enough units to pay for the cut tiles: 128 rows, 6144 x 4096 35 | 40, 4096 x 14336 58 | 54,
     // 28672 x 4096 115 | 81.  To 256 rows the prefill kernel takes one tile and this one two, so only where its limit of
@@ -351,6 +353,7 @@ cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, int
 int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
     int launches = 0;
     cudaError_t e = run_rows(h, a, st, BPQ4K_TYPE_Q4_K, &launches);
+    h->last_kernel = BPQ4K_KERNEL_ROWS;
     if (e != cudaErrorInvalidValue) {
         h->launches += (uint64_t)launches;
         if (e == cudaSuccess) return BPQ4K_OK;
@@ -359,8 +362,10 @@ int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
     }
     e = cudaSuccess;
     if (h->gemv_variant == BPQ4K_GEMV_FP32) {
+        h->last_kernel = BPQ4K_KERNEL_FLOAT;
         e = launch_gemv_fp32(a, st, &launches);
     } else if (!a.n_slots && a.M >= (uint32_t)h->prefill_min_m && h->gemv_variant == BPQ4K_GEMV_AUTO) {
+        h->last_kernel = BPQ4K_KERNEL_PREFILL;
         // prefill: tensor-core kernel; its 16-bit copy of the activations lives in the handle's scratch
         const size_t need = prefill_scratch_bytes(a.M, a.N, a.K, h->prefill_arg(), h->sm_count);
         if (need > h->scratch_bytes) {
@@ -368,6 +373,7 @@ int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
         }
         e = launch_prefill_tc(a, h->prefill_arg(), h->scratch, h->scratch_bytes, h->dev_status, h->sm_count, st, &launches);
     } else {
+        h->last_kernel = BPQ4K_KERNEL_STREAM;
         const uint32_t Mtot = a.n_slots ? 1 : a.M;
         const size_t need = a.n_slots ? 0 : gemv_stream_scratch_bytes(Mtot < kStreamMaxM ? Mtot : kStreamMaxM, a.K);
         if (need > h->scratch_bytes) {
@@ -621,6 +627,7 @@ int bpq4k_get_option(bpq4k_handle_t h, int option, int* value) {
         case BPQ4K_OPT_STREAM_STAMPS: *value = (int)h->tune.stamp_launches; return BPQ4K_OK;
         case BPQ4K_OPT_PREFILL_MIN_M: *value = h->prefill_min_m; return BPQ4K_OK;
         case BPQ4K_OPT_ROWS_MIN_M: *value = h->rows_min_m; return BPQ4K_OK;
+        case BPQ4K_OPT_LAST_MATMUL_KERNEL: *value = h->last_kernel; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_WARPS: *value = (int)h->tune.warps; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_KSPLIT: *value = (int)h->tune.wk; return BPQ4K_OK;
         case BPQ4K_OPT_STREAM_STAGE_BLOCKS: *value = (int)h->tune.cb; return BPQ4K_OK;
@@ -864,6 +871,7 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
     cudaError_t e = cudaErrorInvalidValue;
     if (qtype == BPQ4K_TYPE_Q5_K) {
         e = run_rows(h, a, static_cast<cudaStream_t>(stream), qtype, &launches);
+        h->last_kernel = BPQ4K_KERNEL_ROWS;
         if (e != cudaErrorInvalidValue) {
             h->launches += (uint64_t)launches;
             if (e == cudaSuccess) return BPQ4K_OK;
@@ -871,6 +879,7 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
             return cuda_fail(h, e, "matmul launch");
         }
     }
+    h->last_kernel = BPQ4K_KERNEL_STREAM;
     // many rows of Q5_K or padded Q6_K: the tensor-core kernel, as for Q4_K
     const bool tensor_cores = (qtype == BPQ4K_TYPE_Q5_K || qtype == BPQ4K_TYPE_Q6_K_PADDED) && h->gemv_variant == BPQ4K_GEMV_AUTO &&
                               aligned16(X) && M >= (uint32_t)h->prefill_min_m;
@@ -900,6 +909,7 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
         if (need > h->scratch_bytes) {
             if (int s = ensure_bytes(h, &h->scratch, &h->scratch_bytes, need)) return s;
         }
+        h->last_kernel = BPQ4K_KERNEL_PREFILL;
         e = launch_prefill_tc(a, h->prefill_arg(), h->scratch, h->scratch_bytes, h->dev_status, h->sm_count,
                               static_cast<cudaStream_t>(stream), &launches, qtype);
     } else
@@ -920,7 +930,10 @@ int bpq4k_kq_matmul_f32(bpq4k_handle_t h, int qtype, const float* X, const void*
                                    static_cast<cudaStream_t>(stream), &launches, 13);
         }
     }
-    if (e == cudaErrorInvalidValue) e = launch_kq_gemv_fp32(qtype, a, static_cast<cudaStream_t>(stream), &launches);
+    if (e == cudaErrorInvalidValue) {
+        h->last_kernel = BPQ4K_KERNEL_FLOAT;
+        e = launch_kq_gemv_fp32(qtype, a, static_cast<cudaStream_t>(stream), &launches);
+    }
     h->launches += (uint64_t)launches;
     if (e != cudaSuccess) {
         cudaGetLastError();

@@ -44,6 +44,8 @@ OPT_STREAM_STAMPS = 24
 PREFILL_ONE_CTA, PREFILL_CTA_PAIR, PREFILL_TMEM_WEIGHTS = 0, 1, 2
 OPT_STREAM_UNIT_ROWS = 19
 OPT_BATCH_RECORDS = 30   # read-only: replay graphs recorded by matmul_host_batch
+OPT_LAST_MATMUL_KERNEL = 31   # read-only: which kernel computed the last plain matmul
+KERNEL_NONE, KERNEL_FLOAT, KERNEL_STREAM, KERNEL_PREFILL, KERNEL_ROWS = 0, 1, 2, 3, 4
 GEMV_AUTO, GEMV_FP32, GEMV_STREAM = 0, 1, 2
 PROLOGUE_NONE, PROLOGUE_RMSNORM, PROLOGUE_GELU_MUL, PROLOGUE_SILU_MUL = 0, 1, 2, 3
 PREFILL_F16X3, PREFILL_F16, PREFILL_BF16 = 0, 1, 2

@@ -122,7 +122,10 @@ typedef enum bpq4k_option {
     /* Read-only (bpq4k_get_option): how many times bpq4k_matmul_host_batch_f32 has recorded a dispatch
      * list into a replay graph on this handle.  A list is recorded again after any of the handle's
      * buffers had to grow. */
-    BPQ4K_OPT_BATCH_RECORDS = 30
+    BPQ4K_OPT_BATCH_RECORDS = 30,
+    /* Read-only: which kernel computed the handle's last plain matmul (bpq4k_matmul_f32, bpq4k_kq_matmul_f32 and the
+     * host forms): a bpq4k_matmul_kernel.  The outputs' last bits depend on it. */
+    BPQ4K_OPT_LAST_MATMUL_KERNEL = 31
 } bpq4k_option;
 
 typedef enum bpq4k_gemv_variant {
@@ -130,6 +133,14 @@ typedef enum bpq4k_gemv_variant {
     BPQ4K_GEMV_FP32 = 1,   /* one warp per output row, float FMAs (the reference shader's arithmetic) */
     BPQ4K_GEMV_STREAM = 2  /* bulk-copy ring + tensor-core dot products, split-precision activations */
 } bpq4k_gemv_variant;
+
+typedef enum bpq4k_matmul_kernel {
+    BPQ4K_KERNEL_NONE = 0,
+    BPQ4K_KERNEL_FLOAT = 1,     /* one warp per output row, float FMAs */
+    BPQ4K_KERNEL_STREAM = 2,    /* the streaming kernels */
+    BPQ4K_KERNEL_PREFILL = 3,   /* the tensor-core kernel of BPQ4K_OPT_PREFILL_MODE */
+    BPQ4K_KERNEL_ROWS = 4       /* the several-rows kernel */
+} bpq4k_matmul_kernel;
 
 typedef enum bpq4k_prefill_mode {
     BPQ4K_PREFILL_F16X3 = 0,  /* three-term half split of W and X: meets the float tolerance */

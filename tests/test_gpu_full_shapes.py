@@ -83,7 +83,8 @@ PREFILL_MODES = [(q4k.PREFILL_F16X3, "f16x3", 1e-3, 2e-2), (q4k.PREFILL_F16, "f1
 @pytest.mark.parametrize("mode,name,rel_tol,abs_tol", PREFILL_MODES, ids=[m[1] for m in PREFILL_MODES])
 @pytest.mark.parametrize("N,K", [(14336, 4096), (128256, 4096), (4096, 14336)])
 def test_config2_prefill_m512_row_sample(ctx, N, K, mode, name, rel_tol, abs_tol):
-    """M = 512 through the tensor-core kernel on the whole matrix; the checker computes the sampled rows.  The
+    """M = 512 on the whole matrix, as the library routes it (the float mode: the several-rows kernel; the single-pass
+    modes: the prefill kernel); the checker computes the sampled rows.  The
     three-pass mode is held to the stated tolerance of the path, the single-pass modes to the rounding of their
     16-bit operands (they are outside the tolerance by construction and reported as such)."""
     import torch

@@ -203,7 +203,7 @@ PREFILL_MODES = [(q4k.PREFILL_F16X3, "f16x3"), (q4k.PREFILL_F16, "f16"), (q4k.PR
 
 @pytest.mark.parametrize("mode,name", PREFILL_MODES, ids=[m[1] for m in PREFILL_MODES])
 @pytest.mark.parametrize("M,N,K", [(25, 130, 512), (40, 300, 1024), (64, 256, 256), (100, 130, 512), (256, 300, 1024), (300, 1024, 2048),
-                                   (512, 4096, 4096), (512, 1000, 14336)])
+                                   (512, 4096, 4096), (512, 1000, 14336), (200, 520, 14336), (300, 257, 5120)])
 def test_prefill_tensor_core(ctx, M, N, K, mode, name):
     """Large M goes to the tcgen05 kernel.  The three-pass half split must meet the float tolerance
     of the path; the single-pass modes round weights and activations to 16 bits and are held to the
@@ -213,15 +213,19 @@ def test_prefill_tensor_core(ctx, M, N, K, mode, name):
     raw = synth.make_q4k_weights(N, K, 60)
     x = synth.make_activations(M, K, 61)
     bias = np.linspace(-1, 1, N).astype(np.float32)
+    default_rows = ctx.get_option(q4k.OPT_ROWS_MIN_M)
     ctx.set_option(q4k.OPT_PREFILL_MODE, mode)
+    ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)   # (not the several-rows kernel)
     try:
         w = ctx.upload(pack_q4k(raw, N, K))
         ctx.launch_count(reset=True)
         y = ctx.matmul(dev(torch, x), w, dev(torch, bias))
         torch.cuda.synchronize()
         assert ctx.launch_count() in (2, 3)     # activation cast + tensor-core kernel (+ split-K reduction)
+        assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_PREFILL
         assert ctx.device_status() == 0
     finally:
+        ctx.set_option(q4k.OPT_ROWS_MIN_M, default_rows)
         ctx.set_option(q4k.OPT_PREFILL_MODE, q4k.PREFILL_F16X3)
     y = y.cpu().numpy()
     want = orc.matmul(x, raw, bias, N, K, threads=8)
@@ -275,15 +279,19 @@ def test_prefill_threshold_option(ctx):
     x = synth.make_activations(M, K, 63)
     w = ctx.upload(pack_q4k(raw, N, K))
     want = orc.matmul(x, raw, None, N, K)
-    default_min_m = ctx.get_option(q4k.OPT_PREFILL_MIN_M)
+    default_min_m, default_rows = ctx.get_option(q4k.OPT_PREFILL_MIN_M), ctx.get_option(q4k.OPT_ROWS_MIN_M)
+    ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)   # (not the several-rows kernel)
     ctx.set_option(q4k.OPT_PREFILL_MIN_M, 65)
     ctx.launch_count(reset=True)
     y_stream = ctx.matmul(dev(torch, x), w).cpu().numpy()
     n_stream = ctx.launch_count(reset=True)
+    assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_STREAM
     ctx.set_option(q4k.OPT_PREFILL_MIN_M, 64)
     y_tc = ctx.matmul(dev(torch, x), w).cpu().numpy()
     n_tc = ctx.launch_count()
+    assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_PREFILL
     ctx.set_option(q4k.OPT_PREFILL_MIN_M, default_min_m)
+    ctx.set_option(q4k.OPT_ROWS_MIN_M, default_rows)
     # slabs of 8 or 16 rows (one launch each; two where the activations are quantised by a kernel of their own)
     # vs. cast + tensor-core launch (+ reduction)
     assert n_stream in (4, 8, 16) and n_tc in (2, 3)
@@ -633,6 +641,12 @@ def test_several_rows_with_long_k_walk_k_in_phases(ctx, M, N, K):
     raw = synth.make_q4k_weights(N, K, 90 + M)
     x = synth.make_activations(M, K, 91)
     bias = np.linspace(-3, 3, N).astype(np.float32)
-    y = run_matmul(ctx, x, raw, bias, N, K)
+    default_rows = ctx.get_option(q4k.OPT_ROWS_MIN_M)
+    ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)   # (not the several-rows kernel)
+    try:
+        y = run_matmul(ctx, x, raw, bias, N, K)
+        assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_STREAM
+    finally:
+        ctx.set_option(q4k.OPT_ROWS_MIN_M, default_rows)
     check(y, orc.matmul(x, raw, bias, N, K, threads=8))
     assert ctx.device_status() == 0

@@ -13,7 +13,7 @@ def ctx():
     import backpack_b200 as bp
 
     c = bp.Q4KContext(0)
-    c.set_option(q4k.OPT_ROWS_MIN_M, 2)   # (also the row counts that the streaming kernel serves by default)
+    c.set_option(q4k.OPT_ROWS_MIN_M, 2)   # every call of two rows and more, also those that other kernels serve by default
     yield c
     c.close()
 
@@ -62,10 +62,44 @@ def test_rows_kernel_matches_64_bits(ctx, qtype, M, N, K):
     ctx.launch_count(reset=True)
     y = ctx.matmul(xd, w, bias=bd)
     assert ctx.launch_count() in (2, 3)       # the activations' layout, the matmul, the sum of tiles cut into many segments
+    assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_ROWS
     y2 = ctx.matmul(xd, w, bias=bd)
     assert ctx.device_status() == 0
     close(y.cpu().numpy(), x, w64, bias)
     assert torch.equal(y, y2)                 # cut tiles are summed in a fixed order
+
+
+@pytest.fixture(scope="module", params=[q4k.Q4_K, q4k.Q5_K], ids=["q4_k", "q5_k"])
+def tall(ctx, request):
+    """40003 x 4096: 157 row tiles, 17 super-blocks a CTA, so that each CTA ends one tile and begins another.  Expected
+    values of sampled rows, among them the first and last of a tile and of the matrix."""
+    N, K = 40003, 4096
+    raw = (synth.make_q4k_weights(N, K, 71) if request.param == q4k.Q4_K else synth.make_kq_weights(q4k.Q5_K, N, K, 71)).reshape(N, -1)
+    rows = np.unique(np.concatenate([np.arange(0, N, 256), np.arange(255, N, 256), [N - 1], np.random.default_rng(72).integers(0, N, 300)]))
+    sample = np.ascontiguousarray(raw[rows]).reshape(-1)
+    w64 = orc.dequant(sample, len(rows), K) if request.param == q4k.Q4_K else orc.kq_dequant(orc.Q5_K, sample, len(rows), K)
+    yield upload(ctx, request.param, raw.reshape(-1), N, K), rows, w64.reshape(len(rows), K).astype(np.float64)
+
+
+@pytest.mark.parametrize("M", [6, 16, 23, 32, 47, 64, 80, 96, 112, 128, 250])
+def test_rows_kernel_of_many_units_a_cta(ctx, tall, M):
+    """Rings that wrap, accumulators that alternate, whole tiles inside a share, tiles that two CTAs cut: each activation tile
+    in both types (250 rows: two of 128).  To 48 rows the CTA that ends last adds a cut tile up (two launches), above a
+    launch of its own does."""
+    import torch
+
+    w, rows, w64 = tall
+    x = synth.make_activations(M, w.K, M)
+    xd = torch.from_numpy(x).cuda()
+    ctx.launch_count(reset=True)
+    y = ctx.matmul(xd, w)
+    assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_ROWS
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert ctx.launch_count() == (2 if M <= 48 else 3)
+    y2 = ctx.matmul(xd, w)
+    assert ctx.device_status() == 0
+    close(y[:, torch.from_numpy(rows).cuda()].cpu().numpy(), x, w64)
+    assert torch.equal(y, y2)
 
 
 @pytest.mark.parametrize("M", [7, 20, 40, 64, 90])
@@ -151,7 +185,7 @@ def test_rows_kernel_not_finite_stays_in_its_row(ctx):
 
 def test_rows_kernel_threshold_streams_and_capture(ctx):
     """Below the option's row count the streaming kernel runs; calls on several streams at once keep memory of their own, and
-    each of them runs this kernel (three launches; the streaming kernel takes one); a captured call replays."""
+    each of them runs this kernel; a captured call replays."""
     import torch
 
     M, N, K = 12, 1000, 2048
@@ -161,9 +195,8 @@ def test_rows_kernel_threshold_streams_and_capture(ctx):
     default = ctx.get_option(q4k.OPT_ROWS_MIN_M)
     try:
         ctx.set_option(q4k.OPT_ROWS_MIN_M, M + 1)
-        ctx.launch_count(reset=True)
         close(ctx.matmul(torch.from_numpy(xs[0]).cuda(), w).cpu().numpy(), xs[0], w64)
-        assert ctx.launch_count() == 1
+        assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_STREAM
     finally:
         ctx.set_option(q4k.OPT_ROWS_MIN_M, default)
     xd = [torch.from_numpy(x).cuda() for x in xs]
@@ -171,25 +204,25 @@ def test_rows_kernel_threshold_streams_and_capture(ctx):
     ys = [torch.empty(M, N, device="cuda") for _ in xs]
     streams = [torch.cuda.Stream() for _ in xs]
     torch.cuda.synchronize()
-    ctx.launch_count(reset=True)
     for _ in range(20):
         for x, y, s in zip(xd, ys, streams):
             with torch.cuda.stream(s):
                 ctx.matmul(x, w, out=y)
+                assert ctx.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_ROWS
     torch.cuda.synchronize()
-    assert ctx.launch_count() == 3 * 20 * len(xs)
     for x, y, v in zip(xs, ys, want):
         close(y.cpu().numpy(), x, w64)
         assert torch.equal(y, v)              # whichever stream a call runs on
     import backpack_b200 as bp
 
     c = bp.Q4KContext(0)
+    c.set_option(q4k.OPT_ROWS_MIN_M, 2)
     try:
         y = torch.empty(M, N, device="cuda")
         g = torch.cuda.CUDAGraph()
         with torch.cuda.graph(g):             # the handle's first call
             c.matmul(xd[0], w, out=y)
-        assert c.launch_count() == 3
+        assert c.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_ROWS
         for x in (1, 2):
             xd[0].copy_(xd[x])
             g.replay()
@@ -353,6 +386,7 @@ def test_rows_kernel_first_call_of_a_stream_beside_a_busy_default_stream():
 
     M, N, K = 12, 38400, 1024
     c = bp.Q4KContext(0)
+    c.set_option(q4k.OPT_ROWS_MIN_M, 2)
     try:
         raw = synth.make_q4k_weights(N, K, 31)
         w = c.upload(q4k.pack_q4k(raw, N, K))
