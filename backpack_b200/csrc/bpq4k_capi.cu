@@ -267,32 +267,46 @@ uint8_t* graph_block(bpq4k_context* h, cudaStream_t st, unsigned long long captu
     return mem;
 }
 
-// Which Q4_K / Q5_K calls take the several-rows kernel.  To 8 rows the streaming kernel reads the
-// weights once too and is as fast while their digits fit in shared memory (8 rows, 6144 x 4096 13.3 us against 13.5 here,
-// 128256 x 4096 101 | 97; 9 rows 150 | 97); from K = 8192 on 5 rows do not (5 rows, 57344 x 8192 109 | 88, 8192 x 28672
-// 70 | 50, 4096 x 8192 17 | 16; 4 rows 74 | 88 and 49 | 50).  Below prefill_min_m it stops at 24 rows (a caller who moves the tensor-core threshold up asks for the streaming
-// kernel); at and above the threshold it keeps the float accuracy of the F16X3 mode, so the 16-bit modes, which ask for
-// less, stay with their own kernel.  More than 32 rows of a short K stay with the prefill kernel: from 33 rows on high and
-// low halves share an accumulator, 5.7e-7 of error at any K; the prefill kernel has 3.5e-7 at K = 256, 1.2e-6 at K = 1024.
+// Which Q4_K / Q5_K calls take the several-rows kernel; figures are its speed over the other kernel's on B200, over 1,700
+// timed shapes of 5 to 64 rows (weights from 64 x 256 to 128256 x 28672, both types).
 bool takes_rows_kernel(const bpq4k_context* h, const MatmulArgs& a, int qtype) {
     if (h->gemv_variant != BPQ4K_GEMV_AUTO || a.n_slots || a.n_peers || !aligned16(a.X)) return false;
-    const uint32_t min_m = h->rows_min_m ? (uint32_t)h->rows_min_m : a.K >= 8192u ? 5u : 9u;
-    if (a.M < min_m || a.M > kRowsMaxM || a.K > kRowsMaxK || (a.M > 32u && a.K < 1024u && !h->rows_min_m)) return false;
-    if (a.M < (uint32_t)h->prefill_min_m) return a.M <= 24u;
+    if (a.M > kRowsMaxM || a.K > kRowsMaxK) return false;
+    const bool forced = h->rows_min_m != 0;  // the caller's own threshold, instead of the comparisons below
+    if (a.M < (forced ? (uint32_t)h->rows_min_m : 5u)) return false;
+    if (a.M < (uint32_t)h->prefill_min_m) {
+        // Against the streaming kernel.  A caller who moves the tensor-core threshold up asks for that one above 24 rows.
+        if (a.M > 24u) return false;
+        if (forced) return true;
+        // There a narrow matrix is fast where K splits evenly over eight warps: 1024 x 6144, 5 rows 0.85, but 1024 x 7936 3.8.
+        const bool narrow = a.N < 4096u && a.K % 2048u == 0u;
+        // To 8 rows it reads the weights once too and is as fast while their digits fit beside a ring, to K = 4096
+        // (0.80 to 1.12); above, 6144 x 4608 1.32, 4096 x 6144 1.05, 57344 x 8192 1.15, 4096 x 14336 1.00.  Narrow ones: 0.82 to
+        // 0.94 at K = 6144, 0.86 to 1.03 at 8192 and 1.00 to 1.39 from 14336 on.
+        if (a.M <= 8u) return a.K >= 8192u || (a.K > 4096u && !narrow);
+        // To 16 rows it reads them once to K = 2048, twice above (1.03 to 2.9).  To K = 1024 the launches decide (0.6 to 0.85)
+        // until the weights are large: 16384 x 1024 9 rows 0.99, 16 rows 1.18, 128256 x 1024 9 rows 1.12.  Between, 0.92 to
+        // 1.4, narrow 0.92 to 1.02 to 12 rows.
+        // (Narrow ones whose digits would go through the handle's one scratch, 32768 values and more, stay here although they
+        // are up to 18 % slower: calls that overlap on two streams must not share it.)
+        if (a.M <= 16u) {
+            const uint64_t weights = (uint64_t)a.N * a.K;
+            if (a.K <= 1024u) return weights >= (a.M > 12u ? 1u << 24 : 1u << 26);
+            return a.K > 2048u || !narrow || a.M > 12u;
+        }
+        return true;  // (17 to 24 rows: 0.97 to 4)
+    }
+    // Against the prefill kernel.  The several-rows kernel keeps the float accuracy of the F16X3 mode, so the 16-bit modes,
+    // which ask for less, stay with their own kernel.
     if (h->prefill_mode != BPQ4K_PREFILL_F16X3) return false;
-    if (h->rows_min_m) return true;  // the caller's own threshold
-    // Against the prefill kernel (us, prefill | here).  To 96 rows here: 80 rows, 6144 x 4096 33 | 26, 128256 x 4096 350 | 195.
-    // To 128 rows where a CTA has enough units to pay for the cut tiles: 128 rows, 6144 x 4096 35 | 40, 4096 x 14336 58 | 54,
-    // 28672 x 4096 115 | 81.  To 256 rows the prefill kernel takes one tile and this one two, so only where its limit of
-    // 4096 k per slice makes it cut K: 200 rows, 4096 x 14336 74 | 81, 128256 x 4096 466 | 491, 57344 x 8192 529 | 400.
-    // Above here: 300 rows, 6144 x 4096 69 | 57; 512 rows, 6144 x 4096 96 | 93, 57344 x 8192 1183 | 951.
-    const uint64_t units = (uint64_t)((a.N + 255u) / 256u) * (a.K / BPQ4K_QK_K);
-    // Q5_K, whose larger blocks leave the raw ring one stage per row tile, only to 320 rows: 300 rows, 128256 x 4096
-    // 921 | 866; 512 rows 1251 | 1349, but 57344 x 8192 1188 | 1140.
-    const bool cut_k = a.K > 4096u && a.N >= 16384u;
-    if (a.M <= 96u) return true;
-    if (a.M > 256u) return qtype == BPQ4K_TYPE_Q4_K || a.M <= 320u || cut_k;
-    return a.M <= 128u ? units >= 800u : cut_k;
+    if (forced || a.M <= 32u) return true;  // (0.95 to 3.3)
+    // More rows of a short K stay with the prefill kernel: from 33 rows on high and low halves share an accumulator, 5.7e-7
+    // of error at any K; the prefill kernel has 3.5e-7 at K = 256, 1.2e-6 at K = 1024.
+    if (a.K < 1024u) return false;
+    if (a.M <= 64u) return true;  // (1.14 to 3.3)
+    // Either may be half as fast as the other, as their tiles happen to fill the machine (2048 rows, 2048 x 2048 0.70; 257 rows,
+    // 6144 x 8192 1.64), so models of their times are compared.  Near ties stay here, where the error is smaller.
+    return 0.97 * rows_estimate_us(a.M, a.N, a.K, h->sm_count, qtype) <= prefill_estimate_us(a.M, a.N, a.K, h->sm_count, qtype);
 }
 
 // One call of the several-rows kernel.  cudaErrorInvalidValue: it cannot serve the call (form, shape or memory), and the

@@ -154,6 +154,10 @@ cudaError_t launch_prefill_tc(const MatmulArgs& a, int mode, void* scratch, size
 // cudaErrorInvalidValue: not a shape or form of this kernel.
 constexpr uint32_t kRowsMaxM = 16384, kRowsMaxK = 32768;
 size_t rows_buffer_bytes(uint32_t M, uint32_t K);
+// Microseconds a call takes on this kernel | on the prefill kernel in its three-pass mode, more than 64 rows and K from 1024 on
+// (models of the two kernels' work; see beside them).  Only the comparison of the two is used.
+double rows_estimate_us(uint32_t M, uint32_t N, uint32_t K, int sm_count, int qtype);
+double prefill_estimate_us(uint32_t M, uint32_t N, uint32_t K, int sm_count, int qtype);
 cudaError_t launch_rows_tc(const MatmulArgs& a, void* buffer, size_t buffer_bytes, int* status_dev,
                            int sm_count, TmapCache* tmaps, bool pdl, cudaStream_t stream, int* launches, int qtype = 12);
 

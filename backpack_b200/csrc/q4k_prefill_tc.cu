@@ -1239,6 +1239,17 @@ size_t prefill_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int mode_v, int
     return (mode == 0 ? 2 * one : one) + (z > 1 ? (size_t)z * M * N * 4u : 0);
 }
 
+// Waves of CTAs (one fits an SM), each of them its K slice's super-blocks and the end of its tile (from the fifth wave on the
+// power limit lowers the clock), the partial sums of the slices, the cast of the activations (how the constants were
+// found: rows_estimate_us).
+double prefill_estimate_us(uint32_t M, uint32_t N, uint32_t K, int sm_count, int qtype) {
+    const uint32_t nblk = K / kQK, z = choose_ksplit(M, N, K, 0, sm_count), bps = (nblk + z - 1) / z, tile = choose_tok_tile(M);
+    const uint64_t ctas = (uint64_t)((N + 127u) / 128u) * ((M + tile - 1u) / tile) * z, waves = (ctas + (uint64_t)sm_count - 1u) / (uint64_t)sm_count;
+    const double t = tile / 256.0;
+    return 10.0 + (double)waves * (bps * ((qtype == 13 ? 2.73 : 2.41) + 1.82 * t) + 1.63 * t) +
+           (waves > 4u ? 1.59 * t * (double)(waves - 4u) * bps : 0.0) + (z > 1 ? 1.72e-6 * M * N * z : 0.0) + 0.52e-6 * M * K;
+}
+
 // mode: 0 = three-pass half split, 1 = one pass half, 2 = one pass bfloat16 (the values of bpq4k_prefill_mode)
 cudaError_t launch_prefill_tc(const MatmulArgs& m, int mode_v, void* scratch, size_t scratch_bytes, int* status_dev,
                               int sm_count, cudaStream_t stream, int* launches, int qtype) {

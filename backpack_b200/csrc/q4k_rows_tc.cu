@@ -1030,6 +1030,21 @@ static size_t rows_part_bytes(uint32_t M) {
 }
 size_t rows_buffer_bytes(uint32_t M, uint32_t K) { return rows_head_bytes(M) + rows_image_bytes(M, K) + rows_part_bytes(M); }
 
+// Units of the busiest CTA (a unit's mmas grow with the tile, its dequantisation does not; Q5_K's fifth bit), the ends of its
+// tiles, the segments of cut tiles that are written and read again, the packing of the activations.  Fitted, like the
+// prefill kernel's, to 2,116 timed calls (65 to 2048 rows, weights from 64 x 1024 to 128256 x 4096 and 40960 x 28672, both
+// types; 9 % rms).  The choice between the two misses the faster kernel by more than 6 % for 104 of them, by 20 % at most.
+double rows_estimate_us(uint32_t M, uint32_t N, uint32_t K, int sm_count, int qtype) {
+    const uint32_t T = rows_tile(M), ctas = (uint32_t)sm_count < kMaxCtas ? (uint32_t)sm_count : kMaxCtas;
+    const uint64_t nsb = K / kQK, tiles = (uint64_t)((N + kTileRows - 1u) / kTileRows) * ((M + T - 1u) / T), units = tiles * nsb;
+    const uint64_t grid = units < ctas ? units : ctas, per = (units + grid - 1u) / grid;
+    const uint64_t cuts = units % (grid * nsb) == 0u ? 0u : grid - 1u, segments = cuts + (cuts < tiles ? cuts : tiles);
+    const double t = T / 128.0;
+    const bool q5 = qtype == 13;
+    return 5.5 + (double)per * ((q5 ? 1.54 : 1.33) + (q5 ? 3.95 : 3.54) * t) + 7.3 * t * (double)((per + nsb - 1u) / nsb) +
+           0.91e-6 * (double)segments * (M < T ? M : T) * kTileRows + 1.77e-6 * M * K;
+}
+
 cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_bytes, int* status_dev, int sm_count,
                            TmapCache* tmaps, bool pdl, cudaStream_t stream, int* launches, int qtype) {
     if (m.M == 0 || m.N == 0) return cudaSuccess;

@@ -413,3 +413,31 @@ def test_rows_kernel_first_call_of_a_stream_beside_a_busy_default_stream():
             assert float((y.double() - v).norm() / v.norm()) <= 4e-6
     finally:
         c.close()
+
+
+# Shapes where the two kernels that could serve a call are at least 5 % apart, and the faster one.
+ROUTES = [(4, 6144, 4608, "stream"), (5, 1024, 7936, "rows"), (5, 1024, 6144, "stream"), (8, 6144, 4608, "rows"), (8, 16384, 8192, "rows"),
+          (8, 1024, 4096, "stream"), (8, 256, 28672, "rows"), (9, 256, 2304, "rows"), (9, 16384, 512, "stream"), (12, 1024, 1024, "stream"),
+          (12, 4096, 1024, "stream"), (16, 16384, 1024, "rows"), (16, 8192, 2048, "rows"), (17, 16384, 1024, "rows"), (24, 64, 512, "rows"),
+          (25, 64, 1024, "rows"), (32, 28672, 256, "rows"), (48, 1024, 512, "prefill"), (64, 28672, 1024, "rows"), (97, 256, 2048, "rows"),
+          (128, 16384, 1024, "prefill"), (128, 28672, 4096, "rows"), (200, 10240, 1024, "prefill"), (257, 6144, 8192, "rows"),
+          (512, 16384, 1024, "prefill"), (512, 28672, 8192, "rows"), (1024, 1024, 8192, "prefill"), (2048, 2048, 2048, "prefill")]
+
+
+@pytest.mark.parametrize("M,N,K,kernel", ROUTES)
+def test_calls_take_the_faster_kernel(M, N, K, kernel):
+    import torch
+
+    import backpack_b200 as bp
+
+    if torch.cuda.get_device_properties(0).multi_processor_count != 148:
+        pytest.skip("the routes were timed on 148 SMs")
+    c = bp.Q4KContext(0)
+    try:
+        for qtype, size in ((q4k.Q4_K, 144), (q4k.Q5_K, 176)):
+            w = q4k.Q4KWeight(torch.zeros(N * (K // 256) * size, dtype=torch.uint8, device="cuda"), N, K, (K // 256) * size // 4, qtype)
+            y = c.matmul(torch.ones(M, K, device="cuda"), w)
+            got = {q4k.KERNEL_STREAM: "stream", q4k.KERNEL_PREFILL: "prefill", q4k.KERNEL_ROWS: "rows"}[c.get_option(q4k.OPT_LAST_MATMUL_KERNEL)]
+            assert got == kernel and float(y.abs().max()) == 0.0 and c.device_status() == 0
+    finally:
+        c.close()
