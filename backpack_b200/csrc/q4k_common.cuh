@@ -12,6 +12,15 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+// Debug build (make DEBUG=1 -> libbpq4k_debug.so): index checks compiled into the kernels.  A failed check
+// records kDeviceAssert in the handle's status word and the guarded access is skipped -- never a trap, never a
+// fault.  In the normal build the macro disappears.
+#ifdef BPQ4K_DEBUG_CHECKS
+#define BPQ4K_CHECK(cond, status_ptr) ((cond) ? true : (((status_ptr) ? (void)atomicExch((status_ptr), kDeviceAssert) : (void)0), false))
+#else
+#define BPQ4K_CHECK(cond, status_ptr) (true)
+#endif
+
 namespace bpq4k {
 
 constexpr uint32_t kQK = 256;

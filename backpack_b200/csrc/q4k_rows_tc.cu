@@ -401,6 +401,10 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                 for (uint32_t rt = 0; rt < 2 && ok; rt++) {
                     ok = it == 0 || wait_bar(raw_empty(s), (it - 1u) & 1u, abort_flag, a.status);
                     if (!ok) break;
+                    if (!BPQ4K_CHECK(b < a.nsb && rtile * kTileRows < a.N && s < P::NR, a.status)) {
+                        *abort_flag = 1, ok = false;
+                        break;
+                    }
                     mbar_expect_tx(raw_full(s), P::RAW_BYTES);
                     tma_load_2d(raw_slot(s), &a.tmap_w, b * (P::BLOCK / 4u), rtile * kTileRows + rt * 128u, raw_full(s));
                     issued++;
@@ -423,6 +427,10 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                 for (uint32_t g = 0; g < 4 && ok; g += P::BG) {
                     ok = it == 0 || wait_bar(b_empty(s), (it - 1u) & 1u, abort_flag, a.status);
                     if (!ok) break;
+                    if (!BPQ4K_CHECK(tt < a.tok_tiles && b < a.nsb && s < P::NB, a.status)) {
+                        *abort_flag = 1, ok = false;
+                        break;
+                    }
                     const uint32_t bytes = P::BG * P::G_BYTES + (g + P::BG == 4u ? P::S_BYTES : 0u);
                     mbar_expect_tx(b_full(s), bytes);
                     bulk_load(b_slot(s), src + g * P::G_BYTES, bytes, b_full(s));
@@ -611,7 +619,9 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 #pragma unroll
                         for (uint32_t j = 0; j < 32; j++) {
                             const float r = fmaf(y[j], __shfl_sync(0xFFFFFFFFu, iv, j), bias);
-                            if (c0 + j < tok_n && row_ok) *out = r;
+                            if (c0 + j < tok_n && row_ok &&
+                                BPQ4K_CHECK(whole ? tok0 + c0 + j < a.M && n < a.N : c0 + j < a.slot_rows && blockIdx.x < kMaxCtas, a.status))
+                                *out = r;
                             out += stride;
                         }
                         iv = ivn;
@@ -705,7 +715,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     float* mine = a.part + ((uint64_t)blockIdx.x * 2u + (seg_head ? 1u : 0u)) * slot + t0 * kTileRows + rt * 128u + row;
 #pragma unroll
                     for (int j = 0; j < TH; j++)
-                        if (t0 + j < tok_n) mine[j * kTileRows] = y[j];
+                        if (t0 + j < tok_n && BPQ4K_CHECK(t0 + j < a.slot_rows && blockIdx.x < kMaxCtas, a.status)) mine[j * kTileRows] = y[j];
                     write = false;
                     if (!a.defer) {
                     const uint32_t c_first = unit_owner(dtile * a.nsb, a.u_base, a.u_extra);
@@ -723,7 +733,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                             const float* p = a.part + ((uint64_t)c * 2u + (c == c_first ? 1u : 0u)) * slot + t0 * kTileRows + rt * 128u + row;
 #pragma unroll
                             for (int j = 0; j < TH; j++) {
-                                if (t0 + j < tok_n) y[j] += __ldcg(p + j * kTileRows);
+                                if (t0 + j < tok_n && BPQ4K_CHECK(t0 + j < a.slot_rows && c < gridDim.x, a.status)) y[j] += __ldcg(p + j * kTileRows);
                             }
                         }
                     }
@@ -736,7 +746,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
                     const float* inv = a.inv + tok0 + t0;
 #pragma unroll
                     for (int j = 0; j < TH; j++) {
-                        if (t0 + j < tok_n) *out = fmaf(y[j], __ldcg(inv + j), bias);
+                        if (t0 + j < tok_n && BPQ4K_CHECK(tok0 + t0 + j < a.M, a.status)) *out = fmaf(y[j], __ldcg(inv + j), bias);
                         out += a.N;
                         if (j % 8 == 7) asm volatile("" ::: "memory");
                     }
@@ -835,7 +845,7 @@ __global__ void __launch_bounds__(kThreads, 1) rows_tc_kernel(const __grid_const
 __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict__ X, uint32_t M, uint32_t K, uint32_t T,
                                                         uint8_t* __restrict__ image, float* __restrict__ inv,
                                                         float* __restrict__ sb_scale, uint32_t* __restrict__ spread,
-                                                        uint32_t* __restrict__ counters) {
+                                                        uint32_t* __restrict__ counters, [[maybe_unused]] int* status) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ uint32_t red[8];
@@ -897,6 +907,7 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
         split(e4.y, e4.w, hi.y, lo.y);
         split(o4.x, o4.z, hi.z, lo.z);
         split(o4.y, o4.w, hi.w, lo.w);
+        if (!BPQ4K_CHECK((tt + 1u) * T <= gridDim.y && t < T && sb < nsb, status)) break;
         uint8_t* blk = image + ((uint64_t)tt * nsb + sb) * T * 1088u;
         if (stack && lane == 0) sb_scale[((uint64_t)tt * nsb + sb) * T + t] = live ? __uint_as_float((127u + e - es) << 23) : 0.f;
         auto put = [&](uint32_t r, const uint4& v) { *reinterpret_cast<uint4*>(blk + g * T * 256u + r * 128u + ((i ^ (r & 7u)) << 4)) = v; };
@@ -926,7 +937,7 @@ __global__ void __launch_bounds__(256) rows_pack_kernel(const float* __restrict_
 __global__ void __launch_bounds__(256) rows_reduce_kernel(const float* __restrict__ part, const float* __restrict__ inv,
                                                           const float* __restrict__ bias, float* __restrict__ Y, uint32_t M, uint32_t N,
                                                           uint32_t T, uint32_t tok_tiles, uint32_t slot_rows, uint32_t nsb, uint32_t u_base,
-                                                          uint32_t u_extra) {
+                                                          uint32_t u_extra, [[maybe_unused]] int* status) {
     const uint32_t tile = (unit_begin(blockIdx.x + 1u, u_base, u_extra) - 1u) / nsb;
     const uint32_t rtile = tile / tok_tiles, tok0 = (tile - rtile * tok_tiles) * T;
     const uint32_t t = blockIdx.y * 4u + (threadIdx.x >> 6), r4 = (threadIdx.x & 63u) * 4u, n = rtile * kTileRows + r4;
@@ -934,6 +945,7 @@ __global__ void __launch_bounds__(256) rows_reduce_kernel(const float* __restric
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (c_first != blockIdx.x || c_first == c_last || t >= slot_rows || tok0 + t >= M || n >= N) return;
+    if (!BPQ4K_CHECK(c_last < gridDim.x && c_first < c_last, status)) return;
     const uint64_t slot = (uint64_t)slot_rows * kTileRows;
     const float* p = part + (uint64_t)c_first * 2u * slot + t * kTileRows + r4;
     float4 s = __ldcg(reinterpret_cast<const float4*>(p + slot));
@@ -1116,7 +1128,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     cudaError_t e = cudaLaunchKernelEx(&cfg, rows_pack_kernel, m.X, m.M, m.K, T, const_cast<uint8_t*>(ra.image), const_cast<float*>(ra.inv),
-                                       const_cast<float*>(ra.sb_scale), const_cast<uint32_t*>(ra.spread), ra.counters);
+                                       const_cast<float*>(ra.sb_scale), const_cast<uint32_t*>(ra.spread), ra.counters, status_dev);
     if (launches) ++*launches;
     if (e != cudaSuccess) return e;
     e = q5 ? launch_rows_t<1>(T, ra, grid, pdl, stream) : launch_rows_t<0>(T, ra, grid, pdl, stream);
@@ -1124,7 +1136,7 @@ cudaError_t launch_rows_tc(const MatmulArgs& m, void* buffer, size_t buffer_byte
     if (e != cudaSuccess || !ra.defer) return e;
     cfg.gridDim = dim3(grid, (ra.slot_rows + 3u) / 4u);
     e = cudaLaunchKernelEx(&cfg, rows_reduce_kernel, (const float*)ra.part, ra.inv, ra.bias, ra.Y, ra.M, ra.N, T, tok_tiles, ra.slot_rows, nsb,
-                           ra.u_base, ra.u_extra);
+                           ra.u_base, ra.u_extra, status_dev);
     if (launches) ++*launches;
     return e;
 }

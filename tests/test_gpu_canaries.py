@@ -115,6 +115,27 @@ def test_debug_build_reports_no_failed_index_check(debug_ctx, M, N, K):
     assert debug_ctx.device_status() == 0
 
 
+# several activation rows (q4k_rows_tc.cu): each kind of activation tile, tiles that a CTA adds up at the end, tiles added up
+# by a launch of their own, several activation tiles
+ROWS = [(7, 300, 512), (12, 38400, 1024), (23, 1000, 2560), (32, 3000, 1024), (47, 700, 2048), (64, 130, 4096), (70, 300, 1024), (128, 300, 2048),
+        (300, 520, 1024)]
+
+
+@pytest.mark.parametrize("qtype,layout", [(orc.Q4_K, q4k.Q4_K), (orc.Q5_K, q4k.Q5_K)])
+@pytest.mark.parametrize("M,N,K", ROWS)
+def test_several_rows_stay_inside_their_buffers(ctx, debug_ctx, qtype, layout, M, N, K):
+    """On the product build and on the debug build, whose several-rows kernel checks the coordinates of its copies, its
+    workspace slots and its output indices."""
+    for c in (ctx, debug_ctx):
+        default = c.get_option(q4k.OPT_ROWS_MIN_M)
+        c.set_option(q4k.OPT_ROWS_MIN_M, 2)
+        try:
+            run_guarded_matmul(c, qtype, layout, M, N, K, 800 + M)
+            assert c.get_option(q4k.OPT_LAST_MATMUL_KERNEL) == q4k.KERNEL_ROWS
+        finally:
+            c.set_option(q4k.OPT_ROWS_MIN_M, default)
+
+
 def test_debug_build_fused_and_experts(debug_ctx):
     import torch
 
