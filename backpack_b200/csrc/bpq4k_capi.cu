@@ -361,9 +361,9 @@ cudaError_t run_rows(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st, int
     return e != cudaSuccess ? e : f;
 }
 
-// Kernel selection.  FP32: always the float kernel.  STREAM / AUTO: the streaming
-// kernel, X walked in slabs of 8 rows (each slab re-reads the weights, as the
-// reference's batched8 shader does per 8 rows).
+// Kernel selection.  FP32: always the float kernel.  AUTO: the several-rows kernel where takes_rows_kernel says so, else the
+// prefill kernel from prefill_min_m rows on.  Else, and for STREAM: the streaming kernel, X walked in slabs of 8 rows, 16 to
+// K = 2048 (each slab re-reads the weights, as the reference's batched8 shader does per 8 rows).
 int run_matmul(bpq4k_context* h, const MatmulArgs& a, cudaStream_t st) {
     int launches = 0;
     cudaError_t e = run_rows(h, a, st, BPQ4K_TYPE_Q4_K, &launches);

@@ -1,5 +1,6 @@
-// Prefill Q4_K matmul (M >= 25 by default) on the 5th-generation tensor cores: weights are dequantised
-// on chip into 16-bit tiles, multiplied with tcgen05.mma, accumulated in TMEM.
+// Prefill matmul (M >= 25 by default) on the 5th-generation tensor cores: weights are dequantised on chip into 16-bit tiles,
+// multiplied with tcgen05.mma, accumulated in TMEM.  It serves the single-pass modes, Q6_K, and the three-pass mode of Q4_K and
+// Q5_K where the several-rows kernel (q4k_rows_tc.cu) is slower (takes_rows_kernel).
 //
 // The reference has no tensor-core path for Q4_K: its "prefill" is q4k_matmul_batched8
 // (runtime/kernels/quant_kq/q4k_matmul_batched8.wgsl:9-23, picked at
@@ -10,8 +11,9 @@
 //   Y[m][n] = sum_k X[m][k] * deq(W)[n][k] + bias[n]
 //
 // MMA orientation: D[weight row][activation row] = A[weight row][k] * B[activation row][k]^T, so
-// the 128 TMEM lanes are weight rows and the accumulator columns are activation rows (N_mma = 256).
-// A CTA owns ROWS weight rows (ROWS/128 accumulators of 256 columns) x 256 activation rows and
+// the 128 TMEM lanes are weight rows and the accumulator columns are activation rows (N_mma = 256, or fewer in steps of 16
+// where the rows are shared out over tiles that need not be full).
+// A CTA owns ROWS weight rows (ROWS/128 accumulators of 256 columns) x up to 256 activation rows and
 // walks K in steps of 64 (one 64-weight group of a super-block = one 128-byte swizzle row).
 //
 // Roles (warp-specialised, all hand-offs through mbarriers):
@@ -24,8 +26,8 @@
 //                 (tcgen05.ld), add the bias and store Y.
 //
 // Precision modes: one pass in half or bfloat16 (weights and activations rounded to 16 bits), or
-// three passes with W = Wh + Wl, X = Xh + Xl in half (Wh*Xh + Wh*Xl + Wl*Xh, all into the same
-// accumulator), which meets the float tolerance of the path.
+// three passes with W = Wh + Wl, X = Xh + Xl in half (Wh*Xh, and Wh*Xl + Wl*Xh in an accumulator of their own), which
+// meets the float tolerance of the path.
 //
 // Every wait is bounded: on a time-out the role raises the CTA's abort flag and the device status
 // word, every role leaves its loop, TMEM is freed and the kernel returns.

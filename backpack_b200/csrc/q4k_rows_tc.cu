@@ -14,11 +14,12 @@
 // Error against 64 bits 2.9e-7..3.7e-7 to 32 rows (streaming kernel 3.3e-7..4.5e-7), 5.7e-7..6.3e-7 above (prefill kernel
 // 1.2e-6..2.2e-6 from K = 1024 on).
 //
-// What bounds it.  To 48 rows the instructions of the dequantising warps (3,300 cycles a unit of 256 rows x 256 weights,
-// 1,470 at the DRAM rate; ncu: issue slots 54 % busy, ALU 40 %); above, the hand-overs between dequantising, mma and drain
-// (T = 128: 7,200 cycles a unit, 4,350 of them mmas).  Whole call on B200, us, before | now (before: streaming kernel in
+// What bounds it.  To 48 rows the instructions of the dequantising warps (16 rows: 3,500 cycles a unit of 256 rows x 256
+// weights, 1,470 at the DRAM rate; ncu: issue slots 55 % busy, ALU 41 %, DRAM 32 %); above, the hand-overs between
+// dequantising, mma and drain (T = 128: 8,000 cycles a unit, the tensor pipe busy in 4,300 of them).  Whole call on B200, us, before | now (before: streaming kernel in
 // slabs, prefill kernel with three passes), 128256 x 4096: 16 rows 201 | 105, 24 rows 302 | 115, 37 rows 348 | 147, 64 rows
-// 348 | 159, 80 rows 350 | 195, 128 rows 387 | 267, 512 rows 1252 | 1166; 57344 x 8192, 512 rows: 1183 | 951.
+// 348 | 159, 80 rows 350 | 195, 128 rows 387 | 267, 512 rows 1252 | 1166; 57344 x 8192, 512 rows: 1183 | 951.  The 48- and
+// 128-row variants spill 52 and 112 bytes (128 rows: 2 % of its instructions).
 //   * the dequantised operand lives in TENSOR MEMORY (tcgen05.st, A operand of tcgen05.mma); through shared memory its
 //     write and re-read alone would cost 1.7 times the shared-memory bandwidth that streaming at the DRAM rate leaves;
 //   * a CTA takes 256 weight rows at a time (two 128-lane row tiles share every activation tile);

@@ -68,7 +68,8 @@ typedef enum bpq4k_status {
 typedef enum bpq4k_option {
     BPQ4K_OPT_GEMV_VARIANT = 1,  /* bpq4k_gemv_variant; default AUTO */
     BPQ4K_OPT_PREFILL_MODE = 2,  /* bpq4k_prefill_mode; default F16X3 */
-    BPQ4K_OPT_PREFILL_MIN_M = 3, /* smallest M routed to the tensor-core prefill kernel; default 25 */
+    BPQ4K_OPT_PREFILL_MIN_M = 3, /* smallest M that leaves the streaming kernel for the tensor-core kernels; default 25
+                                  * (Q4_K and Q5_K may take the several-rows kernel from 5 rows on: ROWS_MIN_M) */
     /* Tuning of the streaming kernel; 0 = automatic.  The reference tunes its decode
      * kernels through an autotune cache (runtime/model_runner.cpp:5113-5199). */
     BPQ4K_OPT_STREAM_WARPS = 10,         /* warps per CTA, <= 16 */
@@ -115,9 +116,9 @@ typedef enum bpq4k_option {
      * library with the streaming kernel compiled again) has the stamps; the product library answers n > 0 with
      * BPQ4K_ERR_INVALID_ARG (even untaken, the six branches cost its decode step 2 %).  No counterpart in the reference. */
     BPQ4K_OPT_STREAM_STAMPS = 24,
-    /* Smallest M of Q4_K and Q5_K matmuls that the several-rows kernel serves (K <= 32768).  From BPQ4K_OPT_PREFILL_MIN_M
-     * on it serves the F16X3 mode, below it M <= 24.  Default 0: automatic
-     * (9; 5 from K = 8192 on). */
+    /* Smallest M of Q4_K and Q5_K matmuls that the several-rows kernel serves (K <= 32768, M <= 16384).  From
+     * BPQ4K_OPT_PREFILL_MIN_M on it serves the F16X3 mode only, below it M <= 24.  Default 0: automatic, where it is the
+     * faster kernel (never below 5 rows).  n > 0: every such M from n on; a large n: never. */
     BPQ4K_OPT_ROWS_MIN_M = 25,
     /* Read-only (bpq4k_get_option): how many times bpq4k_matmul_host_batch_f32 has recorded a dispatch
      * list into a replay graph on this handle.  A list is recorded again after any of the handle's
@@ -143,7 +144,8 @@ typedef enum bpq4k_matmul_kernel {
 } bpq4k_matmul_kernel;
 
 typedef enum bpq4k_prefill_mode {
-    BPQ4K_PREFILL_F16X3 = 0,  /* three-term half split of W and X: meets the float tolerance */
+    BPQ4K_PREFILL_F16X3 = 0,  /* float accuracy: the several-rows kernel (two half passes) or a three-term half split of W and
+                               * X, whichever is faster for the shape; |x| < 65504 wherever the latter may serve the call */
     BPQ4K_PREFILL_F16 = 1,    /* single half-precision pass */
     BPQ4K_PREFILL_BF16 = 2    /* single bfloat16 pass */
 } bpq4k_prefill_mode;
@@ -220,8 +222,17 @@ int bpq4k_dequant_f32(bpq4k_handle_t h, const void* W, uint32_t N, uint32_t K,
  * (runtime/model_runner.cpp:2404-2413).  Grid and tile choices are internal.
  * `bias` may be NULL (the reference always binds a zero buffer).  X and W must be
  * 16-byte aligned; Y (outputs are written one float at a time) 4-byte aligned.
- * M >= the PREFILL_MIN_M option goes to the tensor-core kernel in the PREFILL_MODE
- * option's precision; smaller M runs the streaming kernel in slabs of 8 rows. */
+ * Which kernel serves a call follows from its type and shape alone (BPQ4K_OPT_LAST_MATMUL_KERNEL tells): M up to 4 the
+ * streaming kernel; M from 5 on the several-rows kernel (Q4_K and Q5_K) where it is faster; else below PREFILL_MIN_M the
+ * streaming kernel in slabs of 8 rows (16 to K = 2048), from there on the tensor-core kernel in the PREFILL_MODE option's
+ * precision.
+ * Memory: the several-rows kernel takes working memory from a pool of the handle in the stream's order, so calls on
+ * different streams may overlap (16 MB are mapped with the handle, larger calls map more, and the handle keeps twice the
+ * largest).  A captured call has memory of its own, allocated while capturing where needed and used again once the graph,
+ * its executables and their launches are gone: different graphs may run side by side, executables of ONE graph may not (they
+ * share it, as they share Y).  The other kernels' scratch is one per handle: their calls must not overlap on two streams
+ * where they use it (from PREFILL_MIN_M on, and several rows with M rounded up to 4 times K at or above 32768).  All of it is
+ * freed by bpq4k_destroy, after which a graph that holds such a call must not run. */
 int bpq4k_matmul_f32(bpq4k_handle_t h, const float* X, const void* W, const float* bias, float* Y,
                      uint32_t M, uint32_t N, uint32_t K, uint32_t rowStrideWords,
                      uint32_t yOffset, void* stream);
