@@ -125,13 +125,14 @@ def test_rows_kernel_range_of_activations_and_scales(ctx, M):
     y = ctx.matmul(torch.from_numpy(x).cuda(), w).cpu().numpy().astype(np.float64)
     assert ctx.device_status() == 0
     # The kernel splits a weight into sc*(q - 8) and a constant of its sub-block, so a weight that is small beside its
-    # sub-block's largest keeps that one's absolute error: 2^-23 of the activation (2^-39 of the row's largest where that
-    # is more), 16 truncated steps of 2^-23 at most.
+    # sub-block's largest keeps that one's absolute error: 2^-23 of the activation, 16 truncated steps of 2^-23 at most; where
+    # that is more, 2^-39 of the row's largest activation, to 32 rows 2^-47 (2^-36 of a scaled value whose largest is 2^11).
+    floor = 2.0**-39 if M > 32 else 2.0**-47
     wmax = np.repeat(np.abs(w64).reshape(N, K // 32, 32).max(axis=2), 32, axis=1)
     for t in range(M):  # each row by itself: they differ by 60 orders of magnitude
         x64 = x[t].astype(np.float64)
         want = w64 @ x64
-        bound = 4e-6 * (wmax @ np.abs(x64)) + 2.0**-39 * np.abs(x64).max() * wmax.sum(axis=1) + 1e-37
+        bound = 4e-6 * (wmax @ np.abs(x64)) + floor * np.abs(x64).max() * wmax.sum(axis=1) + 1e-37
         assert np.all(np.abs(y[t] - want) <= bound), (t, np.max(np.abs(y[t] - want) / bound))
 
 
